@@ -422,135 +422,214 @@ __global__ void collapse_mask_kernel(V *state, uint64_t count, uint64_t cmask, u
             __stcs(state + i, make_cx<V>(0.0, 0.0));
 }
 
-// <Z> sums. Thread k of the grid (G = gridDim * 256 = 2^gbits threads)
-// visits indices i = it * G + k. Bits of i below gbits are fixed per thread;
-// bits at or above gbits are the bits of `it`. Per block the kernel writes
-// n + 1 partial sums: [0] the block's total, [1 + q] the part with bit q set.
+// <Z> sums: [0] the squared norm, [1 + q] the part with bit q set. A block
+// takes a contiguous range of tiles; in a tile thread t reads kZLoads 16-byte
+// words, word u * 256 + t, all in flight together (one complex128 or two
+// complex64 amplitudes each). Bits of the index inside a word and of u split
+// a thread's own sums, bits of t split the block's sums of thread totals, and
+// bits of the tile number add a tile's total to the sum of each set bit.
+// A large register is bound by HBM reads: 296 blocks of eight 16-byte loads
+// per thread keep 64 KiB per SM in flight, and contiguous tile ranges keep
+// the blocks within one tile of one another (a grid of 512 blocks left the
+// last of its 3.5 blocks per SM alone). Small registers are bound by
+// latency: up to one tile (11 or 12 qubits) one block writes the sums
+// itself; otherwise the second kernel adds the blocks' partials, a warp per
+// sum.
 constexpr int kZThreads = 256;
-constexpr int kZMinBits = 12;                 // registers below this use one thread
-constexpr int kZMaxHi = kMaxQubits - kZMinBits; // "it" bits per thread
+constexpr int kZLoads = 8;
+constexpr int kZMaxBlocks = 296;                // two per SM
+constexpr int kZMaxHi = kMaxQubits - 11;        // bits of the tile number
 
 template <typename V>
-__global__ void zsums_small_kernel(const V *state, int n, double *sums)
+struct ZTile
 {
-    double s[kMaxQubits + 1];
-    for (int j = 0; j <= n; ++j)
-        s[j] = 0.0;
-    for (uint64_t i = 0; i < (1ull << n); ++i)
+    static constexpr int kBits = 11 + (sizeof(V) == 16 ? 0 : 1);   // amplitudes of a tile
+};
+
+// The sums as the host receives them: result in device memory and, when host
+// is not null, in pinned host memory followed by done = seq (as for a
+// measurement).
+struct ZResult
+{
+    double *sums;
+    double *host;
+    volatile unsigned *done;
+    unsigned seq;
+};
+
+__device__ __forceinline__ void zsums_write(const ZResult &r, int j, double v)
+{
+    r.sums[j] = v;
+    if (r.host != nullptr)
     {
-        const double pr = norm2(state[i]);
-        s[0] += pr;
-        for (int q = 0; q < n; ++q)
-            if ((i >> q) & 1)
-                s[1 + q] += pr;
+        r.host[j] = v;
+        __threadfence_system();
     }
-    for (int j = 0; j <= n; ++j)
-        sums[j] = s[j];
 }
 
-template <typename V>
-__global__ void __launch_bounds__(kZThreads) zsums_kernel(const V *state, int n, int gbits, double *partials)
+// after a block-wide barrier behind every zsums_write of the block
+__device__ __forceinline__ void zsums_signal(const ZResult &r)
 {
-    const uint64_t gt = (uint64_t)blockIdx.x * kZThreads + threadIdx.x;
-    const uint64_t G = 1ull << gbits;
-    const uint64_t iters = 1ull << (n - gbits);
-    double total = 0.0;
-    double hi[kZMaxHi];
-    const int nhi = n - gbits;
+    if (threadIdx.x == 0 && r.host != nullptr)
+    {
+        __threadfence_system();
+        *r.done = r.seq;
+    }
+}
+
+__device__ __forceinline__ double2 ld_word(const double2 *p) { return __ldcs(p); }
+__device__ __forceinline__ float4 ld_word(const float2 *p) { return __ldcs(reinterpret_cast<const float4 *>(p)); }
+// squared norms of a word's amplitudes: the word's sum, and the part of its
+// odd amplitude (complex64)
+__device__ __forceinline__ void word_norms(double2 a, double &sum, double &odd)
+{
+    sum = norm2(a);
+    odd = 0.0;
+}
+__device__ __forceinline__ void word_norms(float4 a, double &sum, double &odd)
+{
+    odd = norm2(make_float2(a.z, a.w));
+    sum = norm2(make_float2(a.x, a.y)) + odd;
+}
+
+// partials: [sum][block]; with one block the sums go to r
+template <typename V>
+__global__ void __launch_bounds__(kZThreads, 2) zsums_kernel(const V *state, int n, double *partials, ZResult r)
+{
+    constexpr int kTileBits = ZTile<V>::kBits;
+    constexpr int kWordBits = kTileBits - 11;           // 0 or 1
+    constexpr int kThreadBit = kWordBits;               // thread bits of the index start here
+    constexpr int kLoadBit = kWordBits + 8;             // then the bits of u
+    const int tid = threadIdx.x, w = tid / 32, l = tid % 32;
+    const int nhi = n > kTileBits ? n - kTileBits : 0;
+    const uint64_t tiles = 1ull << nhi;
+    const uint64_t first = tiles * blockIdx.x / gridDim.x, last = tiles * (blockIdx.x + 1) / gridDim.x;
+    // words of the register below one tile
+    const uint32_t words = n >= kTileBits ? kZLoads * kZThreads : (1u << n) >> kWordBits;
+    double total = 0.0, odd = 0.0, ub[3] = {0.0, 0.0, 0.0}, hi[kZMaxHi];
 #pragma unroll
     for (int q = 0; q < kZMaxHi; ++q)
         hi[q] = 0.0;
-    if (nhi >= 4)
+    for (uint64_t tile = first; tile < last; ++tile)
     {
-        // 16 iterations at a time: 16 loads in flight; bits 0..3 of `it` get
-        // their partial sums from fixed index sets, higher bits get the
-        // block's total once
-        for (uint64_t blk = 0; blk < (iters >> 4); ++blk)
+        const V *base = state + (tile << kTileBits);
+        decltype(ld_word(base)) a[kZLoads];
+        if (words == kZLoads * kZThreads)
         {
-            double pr[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                pr[i] = norm2(__ldcs(state + ((blk << 4) + i) * G + gt));
-            double t = 0.0;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                t += pr[i];
-            total += t;
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-            {
-                double s = 0.0;
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if ((i >> b) & 1)
-                        s += pr[i];
-                hi[b] += s;
-            }
-#pragma unroll
-            for (int q = 4; q < kZMaxHi; ++q)
-                if (q < nhi && ((blk >> (q - 4)) & 1))
-                    hi[q] += t;
+            for (int u = 0; u < kZLoads; ++u)
+                a[u] = ld_word(base + ((u * kZThreads + tid) << kWordBits));
         }
-    }
-    else
-    {
-        for (uint64_t it = 0; it < iters; ++it)
+        else
         {
-            const double pr = norm2(__ldcs(state + it * G + gt));
-            total += pr;
 #pragma unroll
-            for (int q = 0; q < kZMaxHi; ++q)
-                if (q < nhi && ((it >> q) & 1))
-                    hi[q] += pr;
+            for (int u = 0; u < kZLoads; ++u)
+                if (u * kZThreads + tid < words)
+                    a[u] = ld_word(base + ((u * kZThreads + tid) << kWordBits));
+                else
+                    a[u] = decltype(ld_word(base)){};
         }
+        double pr[kZLoads], t = 0.0;
+#pragma unroll
+        for (int u = 0; u < kZLoads; ++u)
+        {
+            double o;
+            word_norms(a[u], pr[u], o);
+            odd += o;
+        }
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+        {
+            double s = 0.0;
+#pragma unroll
+            for (int u = 0; u < kZLoads; ++u)
+                if ((u >> b) & 1)
+                    s += pr[u];
+            ub[b] += s;
+        }
+#pragma unroll
+        for (int u = 0; u < kZLoads; ++u)
+            t += pr[u];
+        total += t;
+#pragma unroll
+        for (int q = 0; q < kZMaxHi; ++q)
+            if (q < nhi && ((tile >> q) & 1))
+                hi[q] += t;
     }
-    __shared__ double sh[kZThreads / 32];
-    const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-    auto block_sum = [&](double v) -> double {
-        v = warp_sum(v);
-        __syncthreads();
+    // per warp: the total, its five lane-bit sums, the thread's own splits
+    constexpr int kFixed = 6 + 3 + 1;
+    __shared__ double sh[kFixed + kZMaxHi][kZThreads / 32];
+    auto put = [&](int row, double v) {
+        const double s = warp_sum(v);
         if (l == 0)
-            sh[w] = v;
-        __syncthreads();
-        double t = 0.0;
-        if (threadIdx.x == 0)
-            for (int k = 0; k < kZThreads / 32; ++k)
-                t += sh[k];
-        return t;
+            sh[row][w] = s;
     };
-    double *out = partials + (size_t)blockIdx.x * (n + 1);
-    const double btotal = block_sum(total);
-    if (threadIdx.x == 0)
-        out[0] = btotal;
-    // Low bits: q < gbits. Thread bits (q < 8) mask the per-thread totals;
-    // block bits (8 <= q < gbits) are uniform in the block.
-    const int tbits = gbits < 8 ? gbits : 8;
-    for (int q = 0; q < tbits; ++q)
+    put(0, total);
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+        put(1 + b, ((l >> b) & 1) ? total : 0.0);
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+        put(6 + b, ub[b]);
+    if (kWordBits)
+        put(9, odd);
+#pragma unroll
+    for (int q = 0; q < kZMaxHi; ++q)
+        if (q < nhi)
+            put(kFixed + q, hi[q]);
+    __syncthreads();
+    if (tid <= n)
     {
-        const double v = block_sum(((threadIdx.x >> q) & 1) ? total : 0.0);
-        if (threadIdx.x == 0)
-            out[1 + q] = v;
+        // sum tid: the total, then bit tid - 1 of the index
+        const int q = tid - 1;
+        int row = 0;
+        unsigned warps = 0xffu;
+        if (q >= 0)
+        {
+            if (q < kThreadBit)
+                row = 9;
+            else if (q < kThreadBit + 5)
+                row = 1 + q - kThreadBit;
+            else if (q < kLoadBit)
+                warps = q - kThreadBit == 5 ? 0xaau : q - kThreadBit == 6 ? 0xccu : 0xf0u;
+            else if (q < kTileBits)
+                row = 6 + q - kLoadBit;
+            else
+                row = kFixed + q - kTileBits;
+        }
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < kZThreads / 32; ++k)
+            if ((warps >> k) & 1)
+                s += sh[row][k];
+        if (gridDim.x == 1)
+            zsums_write(r, tid, s);
+        else
+            partials[(size_t)tid * gridDim.x + blockIdx.x] = s;
     }
-    if (threadIdx.x == 0)
-        for (int q = tbits; q < gbits; ++q)
-            out[1 + q] = ((gt >> q) & 1) ? btotal : 0.0;
-    for (int q = 0; q < nhi; ++q)
+    if (gridDim.x == 1)
     {
-        const double v = block_sum(hi[q]);
-        if (threadIdx.x == 0)
-            out[1 + gbits + q] = v;
+        __syncthreads();
+        zsums_signal(r);
     }
 }
 
-__global__ void zsums_final_kernel(const double *partials, int nblocks, int nsums, double *sums)
+__global__ void __launch_bounds__(1024) zsums_final_kernel(const double *partials, int nblocks, int nsums, ZResult r)
 {
-    for (int j = threadIdx.x; j < nsums; j += blockDim.x)
+    const int w = threadIdx.x / 32, l = threadIdx.x % 32;
+    for (int j = w; j < nsums; j += 32)
     {
         double s = 0.0;
-        for (int b = 0; b < nblocks; ++b)
-            s += partials[(size_t)b * nsums + j];
-        sums[j] = s;
+#pragma unroll
+        for (int i = 0; i < (kZMaxBlocks + 31) / 32; ++i)
+            if (l + 32 * i < nblocks)
+                s += __ldcg(partials + (size_t)j * nblocks + l + 32 * i);
+        s = warp_sum(s);
+        if (l == 0)
+            zsums_write(r, j, s);
     }
+    __syncthreads();
+    zsums_signal(r);
 }
 
 // ------------------------------------------------------------ transfers
@@ -771,22 +850,19 @@ int launch_collapse_mask(typename Cx<R>::T *state, int n, uint64_t cmask, uint64
 }
 
 template <typename R>
-int launch_zsums(const typename Cx<R>::T *state, int n, double *partials, double *sums, cudaStream_t stream)
+int launch_zsums(const typename Cx<R>::T *state, int n, double *partials, double *sums, cudaStream_t stream,
+                 double *host, unsigned *done, unsigned seq)
 {
     typedef typename Cx<R>::T V;
-    const int nsums = n + 1;
-    if (n < kZMinBits)
-    {
-        zsums_small_kernel<V><<<1, 1, 0, stream>>>(state, n, sums);
-        QCSB_CUDA(cudaGetLastError());
-        return 1;
-    }
-    // 2^gbits threads in total: at most 512 blocks of 256 threads.
-    const int gbits = n < 17 ? n : 17;
-    const int blocks = 1 << (gbits - 8);
-    zsums_kernel<V><<<blocks, kZThreads, 0, stream>>>(state, n, gbits, partials);
+    const ZResult r{sums, host, done, seq};
+    const int tile_bits = ZTile<V>::kBits;
+    const uint64_t tiles = n > tile_bits ? 1ull << (n - tile_bits) : 1;
+    const unsigned blocks = static_cast<unsigned>(tiles < kZMaxBlocks ? tiles : kZMaxBlocks);
+    zsums_kernel<V><<<blocks, kZThreads, 0, stream>>>(state, n, partials, r);
     QCSB_CUDA(cudaGetLastError());
-    zsums_final_kernel<<<1, 64, 0, stream>>>(partials, blocks, nsums, sums);
+    if (blocks == 1)
+        return 1;
+    zsums_final_kernel<<<1, 1024, 0, stream>>>(partials, static_cast<int>(blocks), n + 1, r);
     QCSB_CUDA(cudaGetLastError());
     return 2;
 }
@@ -852,7 +928,8 @@ int launch_narrow(const double2 *in, uint64_t count, typename Cx<R>::T *out, cud
                                          unsigned *, unsigned *, unsigned, cudaStream_t);                           \
     template int launch_collapse<R>(Cx<R>::T *, int, int, int, cudaStream_t);                                       \
     template int launch_collapse_mask<R>(Cx<R>::T *, int, uint64_t, uint64_t, cudaStream_t);                        \
-    template int launch_zsums<R>(const Cx<R>::T *, int, double *, double *, cudaStream_t);                          \
+    template int launch_zsums<R>(const Cx<R>::T *, int, double *, double *, cudaStream_t, double *, unsigned *,     \
+                                 unsigned);                                                                         \
     template int launch_gather_logical<R>(const Cx<R>::T *, int, const int *, uint64_t, uint64_t, double2 *,        \
                                           cudaStream_t);                                                            \
     template int launch_scatter_logical<R>(Cx<R>::T *, int, const int *, uint64_t, uint64_t, const double2 *,       \

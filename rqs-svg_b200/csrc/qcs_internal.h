@@ -141,9 +141,12 @@ int launch_collapse_mask(typename Cx<R>::T *state, int n, uint64_t cmask, uint64
 
 // sums[0] = sum |a|^2, sums[1 + q] = sum over amplitudes with bit q set of
 // |a|^2 (physical qubits q = 0..n-1). partials must hold
-// 512 * (n + 1) doubles; sums receives n + 1 doubles.
+// 296 * (n + 1) doubles; sums receives n + 1 doubles. host (pinned host
+// memory, or null) receives them too, followed by done = seq, so that the
+// host can wait for them without synchronising the stream.
 template <typename R>
-int launch_zsums(const typename Cx<R>::T *state, int n, double *partials, double *sums, cudaStream_t stream);
+int launch_zsums(const typename Cx<R>::T *state, int n, double *partials, double *sums, cudaStream_t stream,
+                 double *host = nullptr, unsigned *done = nullptr, unsigned seq = 0);
 inline int launch_zsums(const double2 *state, int n, double *partials, double *sums, cudaStream_t stream)
 {
     return launch_zsums<double>(state, n, partials, sums, stream);

@@ -36,8 +36,11 @@ namespace
 
 constexpr uint64_t kStagingAmps = 1ull << 22;   // 64 MiB per staging buffer
 constexpr size_t kScratchReserve = 256ull << 20;
-constexpr size_t kMeasureFlagOffset = 16;   // in the measurement's pinned buffer, after the (P0, P1) result
-constexpr size_t kMeasureHostBytes = 64;
+// the pinned buffer of reduction results: (P0, P1), the completion flag, the
+// <Z> sums
+constexpr size_t kMeasureFlagOffset = 16;
+constexpr size_t kZsumsOffset = 64;
+constexpr size_t kMeasureHostBytes = kZsumsOffset + sizeof(double) * (kMaxQubits + 1);
 
 bool contains(const std::vector<int> &v, int x) { return std::find(v.begin(), v.end(), x) != v.end(); }
 
@@ -510,12 +513,7 @@ void Simulator::flush()
     if (c64() && norm_target_ < 0.0 && opt_tensor_ != 0 && fusion_mode_ != QCS_FUSION_PLAIN)
     {
         // the norm to restore after this flush is the register's norm now
-        stats.kernel_launches += launch_zsums<float>(static_cast<const float2 *>(state_), n_, zsum_partials_,
-                                                     zsum_result_, stream_);
-        double *h = static_cast<double *>(host_pinned_);
-        QCSB_CUDA(cudaMemcpyAsync(h, zsum_result_, sizeof(double), cudaMemcpyDeviceToHost, stream_));
-        QCSB_CUDA(cudaStreamSynchronize(stream_));
-        norm_target_ = h[0];
+        norm_target_ = register_sums()[0];
     }
     const uint64_t tensor_before = stats.tensor_passes;
     const int k = fused_->run(state_, n_, amp_bytes_, pending_, fusion_mode_, stats, timer);
@@ -549,6 +547,41 @@ void Simulator::synchronize()
     fused_->check_device_error();
 }
 
+unsigned *Simulator::result_flag() const
+{
+    return reinterpret_cast<unsigned *>(static_cast<char *>(meas_host_) + kMeasureFlagOffset);
+}
+
+// Waits until the reduction launched with seq has written its result to the
+// pinned buffer: the host spins on the sequence number that follows it (a
+// stream synchronisation costs a few microseconds more per call); past
+// 500 us of spinning it synchronises the stream instead, which also reports
+// any error.
+void Simulator::wait_result(unsigned seq)
+{
+    const volatile unsigned *flag = result_flag();
+    const auto t0 = std::chrono::steady_clock::now();
+    for (unsigned i = 0; *flag != seq; ++i)
+        if ((i & 255u) == 255u && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(500))
+        {
+            QCSB_CUDA(cudaStreamSynchronize(stream_));
+            break;
+        }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    fused_->check_device_error();
+}
+
+// The squared norm and the per-qubit sums (physical qubits) of the register
+// as it is, in the pinned buffer.
+const double *Simulator::register_sums()
+{
+    double *h = reinterpret_cast<double *>(static_cast<char *>(meas_host_) + kZsumsOffset);
+    const unsigned seq = ++measure_seq_;
+    stats.kernel_launches += QCSB_ON_STATE(launch_zsums, n_, zsum_partials_, zsum_result_, stream_, h, result_flag(), seq);
+    wait_result(seq);
+    return h;
+}
+
 int Simulator::measure(int q)
 {
     // reference measure_qubit, src/qcs.cu:2545-2677
@@ -571,25 +604,12 @@ int Simulator::measure(int q)
         cval |= 1ull << perm_l2p_[m];
     }
     const int t = perm_l2p_[q];
-    // (P0, P1) lands directly in pinned host memory, followed by a sequence
-    // number the host spins on (a stream synchronisation costs a few
-    // microseconds more per measurement); past 500 us of spinning it
-    // synchronises the stream instead, which also reports any error
-    double2 *h = static_cast<double2 *>(meas_host_);
-    unsigned *done = reinterpret_cast<unsigned *>(static_cast<char *>(meas_host_) + kMeasureFlagOffset);
+    // (P0, P1) lands directly in pinned host memory, followed by the flag
+    const double2 *h = static_cast<const double2 *>(meas_host_);
     const unsigned seq = ++measure_seq_;
-    stats.kernel_launches += QCSB_ON_STATE(launch_measure_probs, n_, t, cmask, cval, red_partials_, h, red_ticket_,
-                                           done, seq, stream_);
-    const volatile unsigned *flag = done;
-    const auto t0 = std::chrono::steady_clock::now();
-    for (unsigned i = 0; *flag != seq; ++i)
-        if ((i & 255u) == 255u && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(500))
-        {
-            QCSB_CUDA(cudaStreamSynchronize(stream_));
-            break;
-        }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    fused_->check_device_error();
+    stats.kernel_launches += QCSB_ON_STATE(launch_measure_probs, n_, t, cmask, cval, red_partials_,
+                                           static_cast<double2 *>(meas_host_), red_ticket_, result_flag(), seq, stream_);
+    wait_result(seq);
     const double p0 = h->x, p1 = h->y;
     const double sum = p0 + p1;
     std::uniform_real_distribution<double> dist(0, sum);
@@ -875,11 +895,7 @@ void Simulator::expectation_z(double *out, double *norm)
     if (out == nullptr)
         throw std::runtime_error("expectation_z: output pointer must not be NULL");
     flush();
-    stats.kernel_launches += QCSB_ON_STATE(launch_zsums, n_, zsum_partials_, zsum_result_, stream_);
-    double *h = static_cast<double *>(host_pinned_);
-    QCSB_CUDA(cudaMemcpyAsync(h, zsum_result_, sizeof(double) * (n_ + 1), cudaMemcpyDeviceToHost, stream_));
-    QCSB_CUDA(cudaStreamSynchronize(stream_));
-    fused_->check_device_error();
+    const double *h = register_sums();
     const double total = h[0];
     for (int q = 0; q < n_; ++q)
     {

@@ -185,8 +185,11 @@ class Simulator
     double *zsum_result_ = nullptr;
     void *host_pinned_ = nullptr;
     size_t host_pinned_bytes_ = 0;
-    void *meas_host_ = nullptr;   // pinned: (P0, P1) and the completion flag of a measurement
-    unsigned measure_seq_ = 0;    // sequence number of the last measurement's completion flag
+    void *meas_host_ = nullptr;   // pinned: the results of a reduction (measurement, <Z>) and its completion flag
+    unsigned measure_seq_ = 0;    // sequence number of the last reduction's completion flag
+    unsigned *result_flag() const;
+    void wait_result(unsigned seq);
+    const double *register_sums();
     double2 *staging_dev_ = nullptr;
     double2 *staging_host_ = nullptr;
     uint64_t staging_count_ = 0;
