@@ -299,6 +299,43 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// Insertion of zero bits by runs of adjacent operand positions: run i starts
+// above masks[i] = (1 << pos_i) - 1 and is shifts[i] bits long. A chain of
+// measurements that takes the qubits in order has one run, where a loop over
+// its positions would grow with every measured qubit.
+struct ZeroRuns
+{
+    int count;
+    uint8_t shifts[kMaxOps];
+    uint64_t masks[kMaxOps];
+};
+
+__device__ __forceinline__ uint64_t insert_zero_runs(uint64_t g, const ZeroRuns &z)
+{
+    for (int i = 0; i < z.count; ++i)
+    {
+        const uint64_t lo = g & z.masks[i];
+        g = lo | ((g ^ lo) << z.shifts[i]);
+    }
+    return g;
+}
+
+// operand positions: the set bits of `bits`; returns how many
+int fill_runs(uint64_t bits, ZeroRuns &z)
+{
+    const int n = __builtin_popcountll(bits);
+    z.count = 0;
+    while (bits)
+    {
+        const int pos = __builtin_ctzll(bits);
+        const int len = __builtin_ctzll(~(bits >> pos));
+        z.masks[z.count] = (1ull << pos) - 1;
+        z.shifts[z.count++] = static_cast<uint8_t>(len);
+        bits &= ~(((1ull << len) - 1) << pos);
+    }
+    return n;
+}
+
 template <typename R>
 struct ProbParams
 {
@@ -306,8 +343,7 @@ struct ProbParams
     uint64_t ngroups;
     uint64_t cval;
     uint64_t tbit;
-    int nops;
-    uint64_t masks[kMaxOps];
+    ZeroRuns runs;
     double2 *partials;
     double2 *result;      // final (P0, P1); may be mapped host memory
     unsigned *ticket;     // zero between calls
@@ -346,18 +382,40 @@ __device__ __forceinline__ double2 block_sum_partials(const double2 *partials, i
     return make_double2(t0, t1);
 }
 
-// Per-block (sum |a0|^2, sum |a1|^2) over the groups; fixed reduction order,
-// so repeated calls give identical sums. The last block to finish adds the
-// per-block partials and writes (P0, P1) to p.result.
+// Per-block (sum |a0|^2, sum |a1|^2) over the groups; the grid depends on the
+// group count alone and the reduction order is fixed, so repeated calls give
+// identical sums. The last block to finish adds the per-block partials and
+// writes (P0, P1) to p.result. A chain of measurements halves the groups at
+// every step, and most of its reductions are bound by latency: a block per
+// 2048 groups (eight per thread, four of them in flight), and with one block
+// no partials and no ticket.
+constexpr int kProbGroups = 4;   // groups in flight per thread
+
 template <typename R>
 __global__ void __launch_bounds__(kThreads) measure_probs_kernel(const __grid_constant__ ProbParams<R> p)
 {
     double s0 = 0.0, s1 = 0.0;
-    for (uint64_t g = (uint64_t)blockIdx.x * kThreads + threadIdx.x; g < p.ngroups; g += (uint64_t)gridDim.x * kThreads)
+    const uint64_t step = (uint64_t)gridDim.x * kThreads;
+    for (uint64_t g = (uint64_t)blockIdx.x * kThreads + threadIdx.x; g < p.ngroups; g += kProbGroups * step)
     {
-        const uint64_t i0 = insert_zero_bits<kMaxOps>(g, p.masks, p.nops) | p.cval;
-        s0 += norm2(__ldcs(p.state + i0));
-        s1 += norm2(__ldcs(p.state + (i0 | p.tbit)));
+        typename Cx<R>::T a0[kProbGroups], a1[kProbGroups];
+#pragma unroll
+        for (int u = 0; u < kProbGroups; ++u)
+        {
+            a0[u] = a1[u] = make_cx<typename Cx<R>::T>(0.0, 0.0);
+            if (g + u * step < p.ngroups)
+            {
+                const uint64_t i0 = insert_zero_runs(g + u * step, p.runs) | p.cval;
+                a0[u] = __ldcs(p.state + i0);
+                a1[u] = __ldcs(p.state + (i0 | p.tbit));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kProbGroups; ++u)
+        {
+            s0 += norm2(a0[u]);
+            s1 += norm2(a1[u]);
+        }
     }
     __shared__ double sh[2][kThreads / 32];
     s0 = warp_sum(s0);
@@ -369,29 +427,33 @@ __global__ void __launch_bounds__(kThreads) measure_probs_kernel(const __grid_co
         sh[1][w] = s1;
     }
     __syncthreads();
+    double2 total = make_double2(0.0, 0.0);
     if (threadIdx.x == 0)
-    {
-        double t0 = 0.0, t1 = 0.0;
         for (int k = 0; k < kThreads / 32; ++k)
         {
-            t0 += sh[0][k];
-            t1 += sh[1][k];
+            total.x += sh[0][k];
+            total.y += sh[1][k];
         }
-        p.partials[blockIdx.x] = make_double2(t0, t1);
+    if (gridDim.x > 1)
+    {
+        __shared__ bool last;
+        if (threadIdx.x == 0)
+        {
+            p.partials[blockIdx.x] = total;
+            __threadfence();
+            last = atomicAdd(p.ticket, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last)
+            return;
         __threadfence();
+        total = block_sum_partials(p.partials, gridDim.x);
+        if (threadIdx.x == 0)
+            *p.ticket = 0;
     }
-    __shared__ bool last;
-    if (threadIdx.x == 0)
-        last = atomicAdd(p.ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last)
-        return;
-    __threadfence();
-    const double2 total = block_sum_partials(p.partials, gridDim.x);
     if (threadIdx.x == 0)
     {
         *p.result = total;
-        *p.ticket = 0;
         if (p.done != nullptr)
         {
             // the result reaches host memory before the flag does
@@ -400,7 +462,6 @@ __global__ void __launch_bounds__(kThreads) measure_probs_kernel(const __grid_co
         }
     }
 }
-
 
 template <typename V>
 __global__ void collapse_kernel(V *state, uint64_t ngroups, uint64_t lowmask, uint64_t zero_bit)
@@ -809,12 +870,7 @@ int launch_measure_probs(const typename Cx<R>::T *state, int n, int t, uint64_t 
     ProbParams<R> p;
     std::memset(&p, 0, sizeof(p));
     p.state = state;
-    GateOp op;
-    op.nt = 1;
-    op.tq[0] = t;
-    op.cmask = cmask;
-    p.nops = fill_masks(op, p.masks);
-    p.ngroups = 1ull << (n - p.nops);
+    p.ngroups = 1ull << (n - fill_runs(cmask | (1ull << t), p.runs));
     p.cval = cval;
     p.tbit = 1ull << t;
     p.partials = partials;
@@ -822,8 +878,7 @@ int launch_measure_probs(const typename Cx<R>::T *state, int n, int t, uint64_t 
     p.ticket = ticket;
     p.done = done;
     p.seq = seq;
-    // A fixed grid (independent of n) keeps the partial count constant.
-    measure_probs_kernel<R><<<kReduceBlocks, kThreads, 0, stream>>>(p);
+    measure_probs_kernel<R><<<grid_for(p.ngroups, kThreads * 2 * kProbGroups, kReduceBlocks), kThreads, 0, stream>>>(p);
     QCSB_CUDA(cudaGetLastError());
     return 1;
 }
