@@ -176,11 +176,14 @@ int launch_gather_indices(const typename Cx<R>::T *state, const uint64_t *physic
 int launch_compare(const double2 *x, const double2 *y, uint64_t count, double *partials, cudaStream_t stream);
 
 // Shot sampler (chain rule over physical qubits in the order given by
-// order[0..n)). See sampler.cu for the data layout.
+// order[0..n)): the tree of marginals, then num_shots walks down it. See sampler.cu for the data layout.
 template <typename R>
-int launch_sampler(const typename Cx<R>::T *state, int n, const int *order, uint32_t num_shots,
-                   const double *uniforms, uint64_t *out_bits, double *tree, int split,
-                   cudaStream_t stream);
+int launch_sampler_tree(const typename Cx<R>::T *state, int n, const int *order, double *tree, int split,
+                        cudaStream_t stream);
+template <typename R>
+int launch_sampler_shots(const typename Cx<R>::T *state, int n, const int *order, uint32_t num_shots,
+                         const double *uniforms, uint64_t *out_bits, const double *tree, int split,
+                         cudaStream_t stream);
 size_t sampler_tree_bytes(int n, int *split_out);
 
 } // namespace qcsb

@@ -917,25 +917,20 @@ void Simulator::sample(uint32_t num_shots, uint64_t *out)
     int split = 0;
     const size_t tree_bytes = sampler_tree_bytes(n_, &split);
     const size_t nu = (size_t)num_shots * n_;
-    const size_t need_host = std::max(sizeof(double) * nu, sizeof(uint64_t) * (size_t)num_shots);
-    if (need_host > host_pinned_bytes_)
+    const size_t u_bytes = sizeof(double) * nu, bits_bytes = sizeof(uint64_t) * (size_t)num_shots;
+    if (u_bytes + bits_bytes > host_pinned_bytes_)
     {
         QCSB_CUDA(cudaStreamSynchronize(stream_));
         QCSB_CUDA(cudaFreeHost(host_pinned_));
         host_pinned_ = nullptr;
-        host_pinned_bytes_ = need_host;
-        QCSB_CUDA(cudaMallocHost(&host_pinned_, host_pinned_bytes_));
+        host_pinned_bytes_ = 0;
+        QCSB_CUDA(cudaMallocHost(&host_pinned_, u_bytes + bits_bytes));
+        host_pinned_bytes_ = u_bytes + bits_bytes;
     }
-    double *u = static_cast<double *>(host_pinned_);
-    // same draws, in the same order, as num_shots rounds of measuring
-    // qubits 0..n-1 (src/qcs.cu:2615-2617)
-    std::uniform_real_distribution<double> dist(0.0, 1.0);
-    for (size_t k = 0; k < nu; ++k)
-        u[k] = dist(engine_);
     // one device buffer: tree, then uniforms, then outcomes (256-byte aligned)
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t u_off = up(tree_bytes), bits_off = u_off + up(sizeof(double) * std::max<size_t>(nu, 1));
-    const size_t need_dev = bits_off + up(sizeof(uint64_t) * std::max<uint32_t>(num_shots, 1));
+    const size_t u_off = up(tree_bytes), bits_off = u_off + up(std::max<size_t>(u_bytes, 8));
+    const size_t need_dev = bits_off + up(std::max<size_t>(bits_bytes, 8));
     if (need_dev > sampler_bytes_)
     {
         QCSB_CUDA(cudaStreamSynchronize(stream_));
@@ -949,13 +944,22 @@ void Simulator::sample(uint32_t num_shots, uint64_t *out)
     double *tree = reinterpret_cast<double *>(base);
     double *u_dev = reinterpret_cast<double *>(base + u_off);
     uint64_t *bits_dev = reinterpret_cast<uint64_t *>(base + bits_off);
-    QCSB_CUDA(cudaMemcpyAsync(u_dev, u, sizeof(double) * nu, cudaMemcpyHostToDevice, stream_));
-    stats.kernel_launches += QCSB_ON_STATE(launch_sampler, n_, perm_l2p_.data(), num_shots, u_dev, bits_dev, tree, split, stream_);
-    QCSB_CUDA(cudaStreamSynchronize(stream_));   // the pinned buffer is reused below
-    QCSB_CUDA(cudaMemcpyAsync(host_pinned_, bits_dev, sizeof(uint64_t) * num_shots, cudaMemcpyDeviceToHost, stream_));
+    // the GPU builds the tree while the host draws the uniforms
+    stats.kernel_launches += QCSB_ON_STATE(launch_sampler_tree, n_, perm_l2p_.data(), tree, split, stream_);
+    // same draws, in the same order, as num_shots rounds of measuring
+    // qubits 0..n-1 (src/qcs.cu:2615-2617)
+    double *u = static_cast<double *>(host_pinned_);
+    std::uniform_real_distribution<double> dist(0.0, 1.0);
+    for (size_t k = 0; k < nu; ++k)
+        u[k] = dist(engine_);
+    QCSB_CUDA(cudaMemcpyAsync(u_dev, u, u_bytes, cudaMemcpyHostToDevice, stream_));
+    stats.kernel_launches += QCSB_ON_STATE(launch_sampler_shots, n_, perm_l2p_.data(), num_shots, u_dev, bits_dev, tree,
+                                           split, stream_);
+    uint64_t *bits_host = reinterpret_cast<uint64_t *>(static_cast<char *>(host_pinned_) + u_bytes);
+    QCSB_CUDA(cudaMemcpyAsync(bits_host, bits_dev, bits_bytes, cudaMemcpyDeviceToHost, stream_));
     QCSB_CUDA(cudaStreamSynchronize(stream_));
     fused_->check_device_error();
-    std::memcpy(out, host_pinned_, sizeof(uint64_t) * num_shots);
+    std::memcpy(out, bits_host, bits_bytes);
 }
 
 KernelTimer::~KernelTimer()
