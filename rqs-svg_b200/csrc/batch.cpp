@@ -24,8 +24,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
-#include <thread>
 
 namespace qcsb
 {
@@ -50,24 +48,30 @@ uint64_t dbits(double x)
     return u;
 }
 
-// The GateOp of an actual parameter set laid over the shape's active set.
-GateOp op_like(const GateOp &shape, const GateMatrix &g)
+// Formula of a gate with parameters on the GPU (B_CONST: none needed).
+BatchFormula formula_of(const char *name, int np)
 {
-    GateOp op = shape;
-    const int d = 1 << g.nt;
-    if (shape.diag)
+    static const struct
     {
-        for (int a = 0; a < shape.na; ++a)
-            op.mat[a] = g.m[shape.act[a] * d + shape.act[a]];
-    }
-    else
-    {
-        for (int a = 0; a < shape.na; ++a)
-            for (int b = 0; b < shape.na; ++b)
-                op.mat[a * shape.na + b] = g.m[shape.act[a] * d + shape.act[b]];
-    }
-    return op;
+        const char *name;
+        BatchFormula formula;
+    } table[] = {
+        {"global_phase", B_GLOBAL_PHASE}, {"rx", B_RX}, {"ry", B_RY}, {"rz", B_RZ}, {"u1", B_P}, {"p", B_P},
+        {"u2", B_U2}, {"u3", B_U3}, {"u", B_U3}, {"u4", B_U4}, {"r", B_R}, {"rxx", B_RXX}, {"ryy", B_RYY},
+        {"rzz", B_RZZ}, {"rzx", B_RZX}, {"xx_plus_yy", B_XX_PLUS_YY}, {"xx_minus_yy", B_XX_MINUS_YY},
+    };
+    if (np == 0)
+        return B_CONST;
+    for (const auto &t : table)
+        if (std::strcmp(t.name, name) == 0)
+            return t.formula;
+    throw std::runtime_error(strformat("batch: gate '%s' has no formula on the GPU", name));
 }
+
+// Entries of a parametrised gate stand for themselves while a recipe is made:
+// kTag + 16 gate + element, beyond any constant entry (those are at most 1 in
+// magnitude).
+constexpr double kTag = 4.0;
 
 constexpr size_t kBatchTensorMatsBytes = size_t(2) << 30;   // stage matrices of one batched tensor pass
 
@@ -109,6 +113,14 @@ void Batch::release_device()
     execs_.clear();
     cudaFree(arena_);
     cudaFree(mats_dev_);
+    cudaFree(params_dev_);
+    cudaFree(fill_regs_dev_);
+    cudaFree(recipes_dev_);
+    cudaFree(consts_dev_);
+    params_dev_ = nullptr;
+    fill_regs_dev_ = nullptr;
+    recipes_dev_ = nullptr;
+    consts_dev_ = nullptr;
     cudaFree(zitems_dev_);
     cudaFree(zregs_dev_);
     cudaFree(zpartials_dev_);
@@ -116,12 +128,13 @@ void Batch::release_device()
     cudaFree(tmats_dev_);
     tmats_dev_ = nullptr;
     tmats_bytes_ = 0;
-    if (mats_host_)
-        cudaFreeHost(mats_host_);
+    if (params_host_)
+        cudaFreeHost(params_host_);
+    params_host_ = nullptr;
     if (zout_host_)
         cudaFreeHost(zout_host_);
     arena_ = nullptr;
-    mats_dev_ = mats_host_ = nullptr;
+    mats_dev_ = nullptr;
     zitems_dev_ = nullptr;
     zregs_dev_ = nullptr;
     zpartials_dev_ = zout_dev_ = zout_host_ = nullptr;
@@ -146,7 +159,8 @@ uint32_t Batch::add_circuit(int n, const qcs_b200_gate *gates, uint32_t count)
     Circuit c;
     c.n = n;
     c.gates.reserve(count);
-    uint64_t params = 0;
+    c.param_off = params_.size();
+    std::vector<double> params;
     for (uint32_t i = 0; i < count; ++i)
     {
         const qcs_b200_gate &in = gates[i];
@@ -184,31 +198,24 @@ uint32_t Batch::add_circuit(int n, const qcs_b200_gate *gates, uint32_t count)
                     g.cval |= 1ull << q;
             }
         }
-        for (int j = 0; j < g.np; ++j)
-            g.params[j] = in.params[j];
-        params += g.np;
+        params.insert(params.end(), in.params, in.params + g.np);
         c.gates.push_back(g);
     }
     invalidate();
     circuits_.push_back(std::move(c));
-    num_params_ += params;
+    params_.insert(params_.end(), params.begin(), params.end());
     return static_cast<uint32_t>(circuits_.size() - 1);
 }
 
 void Batch::set_parameters(const double *params, uint64_t count)
 {
-    if (count != num_params_)
+    if (count != params_.size())
         throw std::runtime_error(strformat("set_parameters: the batch has %llu parameters, got %llu",
-                                           (unsigned long long)num_params_, (unsigned long long)count));
+                                           (unsigned long long)params_.size(), (unsigned long long)count));
     if (count > 0 && params == nullptr)
         throw std::runtime_error("set_parameters: params must not be NULL");
-    uint64_t i = 0;
-    for (Circuit &c : circuits_)
-        for (Gate &g : c.gates)
-            for (int j = 0; j < g.np; ++j)
-                g.params[j] = params[i++];
-    // the entries are filled by the next run, group by group, while the GPU
-    // runs the groups before
+    std::copy(params, params + count, params_.begin());
+    // the entries are evaluated by the next run
     dirty_ = built_;
 }
 
@@ -282,6 +289,58 @@ void Batch::plan_group(Group &g, int k, bool tensor)
         }
     }
     g.stride = off;
+    make_recipe(g);
+}
+
+// What every entry of a register's block is: the entry functions run on ops
+// whose parametrised elements are tags.
+void Batch::make_recipe(Group &g)
+{
+    const Circuit &rep = circuits_[g.members.front()];
+    std::vector<GateOp> ops = g.shape;
+    std::vector<uint32_t> param_of(ops.size());
+    uint32_t params = 0;
+    for (size_t i = 0; i < ops.size(); ++i)
+    {
+        param_of[i] = params;
+        params += static_cast<uint32_t>(rep.gates[i].np);
+        if (rep.gates[i].np == 0)
+            continue;
+        GateOp &op = ops[i];
+        for (int a = 0; a < op.na; ++a)
+            for (int b = 0; b < (op.diag ? 1 : op.na); ++b)
+                op.mat[op.diag ? a : a * op.na + b] =
+                    cplx{kTag + 16.0 * static_cast<double>(i) + 4 * op.act[a] + op.act[op.diag ? a : b], 0.0};
+    }
+    g.recipe.assign(g.stride, BatchEntry{B_CONST, 0, 0, 0});
+    g.consts.assign(1, make_double2(0.0, 0.0));
+    double2 m[16];
+    for (const Pass &p : g.passes)
+        for (int f = 0; f < p.prm.nops; ++f)
+        {
+            const FOp &op = p.prm.ops[f];
+            if (op.kind == F_SIGNT)
+                continue;
+            const int ne = layer_kind(op.kind) ? layer_entries(ops, p.src[f], op.kind, m)
+                                               : fop_entries(ops[p.src[f].op], op, p.src[f].swapped, m);
+            for (int e = 0; e < ne; ++e)
+            {
+                BatchEntry &r = g.recipe[op.moff + e];
+                if (m[e].x >= kTag)
+                {
+                    const uint64_t tag = static_cast<uint64_t>(m[e].x - kTag);
+                    const Gate &gt = rep.gates[tag / 16];
+                    r = BatchEntry{formula_of(gt.name, gt.np), static_cast<uint8_t>(tag % 16), 0, param_of[tag / 16]};
+                    continue;
+                }
+                uint32_t ci = 0;
+                while (ci < g.consts.size() && std::memcmp(&g.consts[ci], &m[e], sizeof(double2)) != 0)
+                    ++ci;
+                if (ci == g.consts.size())
+                    g.consts.push_back(m[e]);
+                r.index = ci;
+            }
+        }
 }
 
 void Batch::layout_entries()
@@ -297,13 +356,9 @@ void Batch::layout_entries()
         if (stream_)
             QCSB_CUDA(cudaStreamSynchronize(stream_));
         cudaFree(mats_dev_);
-        if (mats_host_)
-            cudaFreeHost(mats_host_);
-        mats_dev_ = mats_host_ = nullptr;
+        mats_dev_ = nullptr;
         mats_count_ = off;
-        const size_t bytes = sizeof(double2) * std::max<uint64_t>(off, 1);
-        QCSB_CUDA(cudaMalloc(&mats_dev_, bytes));
-        QCSB_CUDA(cudaMallocHost(&mats_host_, bytes));
+        QCSB_CUDA(cudaMalloc(&mats_dev_, sizeof(double2) * std::max<uint64_t>(off, 1)));
     }
     for (Group &g : groups_)
         for (Pass &p : g.passes)
@@ -313,79 +368,56 @@ void Batch::layout_entries()
         }
 }
 
-void Batch::fill_group_range(const Group &g, size_t first, size_t last)
+// The recipes, constants and fill list of the current plans, to the device.
+void Batch::upload_recipes()
 {
-    std::vector<GateOp> ops(g.shape.size());
-    for (size_t s = first; s < last; ++s)
+    std::vector<BatchFillReg> regs;
+    std::vector<BatchEntry> recipes;
+    std::vector<double2> consts;
+    for (Group &g : groups_)
     {
-        const Circuit &c = circuits_[g.members[s]];
-        for (size_t i = 0; i < c.gates.size(); ++i)
-        {
-            const Gate &gt = c.gates[i];
-            ops[i] = op_like(g.shape[i], gate_matrix(gt.id, gt.params, gt.np));
-        }
-        double2 *block = mats_host_ + g.mats_off + (uint64_t)s * g.stride;
-        for (const Pass &p : g.passes)
-            for (int f = 0; f < p.prm.nops; ++f)
-            {
-                const FOp &op = p.prm.ops[f];
-                if (op.kind == F_SIGNT)
-                    continue;
-                if (layer_kind(op.kind))
-                    layer_entries(ops, p.src[f], op.kind, block + op.moff);
-                else
-                    fop_entries(ops[p.src[f].op], op, p.src[f].swapped, block + op.moff);
-            }
-        if (amp_bytes_ == (int)sizeof(float2))
-            entries_to_float(block, g.stride);
+        g.first_reg = static_cast<uint32_t>(regs.size());
+        for (size_t s = 0; s < g.members.size(); ++s)
+            regs.push_back({g.mats_off + (uint64_t)s * g.stride, circuits_[g.members[s]].param_off,
+                            static_cast<uint32_t>(recipes.size()), g.stride, static_cast<uint32_t>(consts.size()), 0});
+        recipes.insert(recipes.end(), g.recipe.begin(), g.recipe.end());
+        consts.insert(consts.end(), g.consts.begin(), g.consts.end());
     }
+    if (stream_)
+        QCSB_CUDA(cudaStreamSynchronize(stream_));
+    cudaFree(fill_regs_dev_);
+    cudaFree(recipes_dev_);
+    cudaFree(consts_dev_);
+    fill_regs_dev_ = nullptr;
+    recipes_dev_ = nullptr;
+    consts_dev_ = nullptr;
+    QCSB_CUDA(cudaMalloc(&fill_regs_dev_, sizeof(BatchFillReg) * regs.size()));
+    QCSB_CUDA(cudaMalloc(&recipes_dev_, sizeof(BatchEntry) * std::max<size_t>(recipes.size(), 1)));
+    QCSB_CUDA(cudaMalloc(&consts_dev_, sizeof(double2) * consts.size()));
+    QCSB_CUDA(cudaMemcpy(fill_regs_dev_, regs.data(), sizeof(BatchFillReg) * regs.size(), cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpy(recipes_dev_, recipes.data(), sizeof(BatchEntry) * recipes.size(), cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpy(consts_dev_, consts.data(), sizeof(double2) * consts.size(), cudaMemcpyHostToDevice));
 }
 
-void Batch::fill_entries(int only_group)
+void Batch::upload_params()
 {
-    // work units: (group, slot range); spread over the host's cores
-    struct Unit
+    // the pinned copy is free again: every run ends with a synchronisation
+    std::copy(params_.begin(), params_.end(), params_host_);
+    QCSB_CUDA(cudaMemcpyAsync(params_dev_, params_host_, sizeof(double) * params_.size(), cudaMemcpyHostToDevice, stream_));
+}
+
+int Batch::fill_entries(int only_group)
+{
+    uint32_t first = 0, count = static_cast<uint32_t>(circuits_.size());
+    if (only_group >= 0)
     {
-        int group;
-        size_t first, last;
-    };
-    std::vector<Unit> units;
-    for (int gi = 0; gi < (int)groups_.size(); ++gi)
-    {
-        if (only_group >= 0 && gi != only_group)
-            continue;
-        const size_t m = groups_[gi].members.size();
-        const size_t step = 64;
-        for (size_t a = 0; a < m; a += step)
-            units.push_back({gi, a, std::min(m, a + step)});
+        first = groups_[only_group].first_reg;
+        count = static_cast<uint32_t>(groups_[only_group].members.size());
     }
-    unsigned hw = std::thread::hardware_concurrency();
-    const unsigned workers = std::max(1u, std::min<unsigned>(hw ? hw : 1, std::min<size_t>(units.size(), 64)));
-    if (workers <= 1)
-    {
-        for (const Unit &u : units)
-            fill_group_range(groups_[u.group], u.first, u.last);
-        return;
-    }
-    std::vector<std::thread> pool;
-    std::vector<std::exception_ptr> errors(workers);
-    for (unsigned w = 0; w < workers; ++w)
-        pool.emplace_back([&, w] {
-            try
-            {
-                for (size_t i = w; i < units.size(); i += workers)
-                    fill_group_range(groups_[units[i].group], units[i].first, units[i].last);
-            }
-            catch (...)
-            {
-                errors[w] = std::current_exception();
-            }
-        });
-    for (auto &t : pool)
-        t.join();
-    for (auto &e : errors)
-        if (e)
-            std::rethrow_exception(e);
+    return amp_bytes_ == 8 ? launch_batch_fill<float>(fill_regs_dev_ + first, count, recipes_dev_, consts_dev_, params_dev_,
+                                                      mats_dev_, stream_)
+                           : launch_batch_fill<double>(fill_regs_dev_ + first, count, recipes_dev_, consts_dev_, params_dev_,
+                                                       mats_dev_, stream_);
 }
 
 // The stage-matrix buffer: the largest tensor pass's matrices over all its
@@ -458,12 +490,7 @@ void Batch::enqueue_passes(const Group &g, cudaStream_t s, int *launches)
 
 void Batch::enqueue_group(int gi, cudaStream_t s, int *launches)
 {
-    const Group &g = groups_[gi];
-    const size_t count = (size_t)g.stride * g.members.size();
-    if (count > 0)
-        QCSB_CUDA(cudaMemcpyAsync(mats_dev_ + g.mats_off, mats_host_ + g.mats_off, sizeof(double2) * count,
-                                  cudaMemcpyHostToDevice, s));
-    enqueue_passes(g, s, launches);
+    enqueue_passes(groups_[gi], s, launches);
 }
 
 void Batch::enqueue_results(cudaStream_t s, int *launches)
@@ -511,9 +538,8 @@ void Batch::tune()
             plan_group(g, cand.first, cand.second);
             layout_entries();
             ensure_tensor_mats();
+            upload_recipes();
             fill_entries(gi);
-            QCSB_CUDA(cudaMemcpyAsync(mats_dev_ + g.mats_off, mats_host_ + g.mats_off,
-                                      sizeof(double2) * g.stride * g.members.size(), cudaMemcpyHostToDevice, stream_));
             int launches = 0;
             enqueue_passes(g, stream_, &launches);   // warm-up
             QCSB_CUDA(cudaEventRecord(ev0_, stream_));
@@ -555,7 +581,7 @@ void Batch::build()
         {
             const GateMatrix gm = gate_matrix(gt.id, kProbe, gt.np);
             const GateOp op = make_gate_op(gm, gt.tq, gt.cmask, gt.cval);
-            sig = mix(sig, (uint64_t)op.nt | ((uint64_t)op.na << 8) | ((uint64_t)op.diag << 16));
+            sig = mix(sig, (uint64_t)op.nt | ((uint64_t)op.na << 8) | ((uint64_t)op.diag << 16) | ((uint64_t)gt.np << 24));
             for (int i = 0; i < op.nt; ++i)
                 sig = mix(sig, (uint64_t)op.tq[i]);
             sig = mix(mix(sig, op.cmask), op.cval);
@@ -628,6 +654,11 @@ void Batch::build()
     QCSB_CUDA(cudaMemcpy(zitems_dev_, items.data(), sizeof(BatchZItem) * items.size(), cudaMemcpyHostToDevice));
     QCSB_CUDA(cudaMemcpy(zregs_dev_, regs.data(), sizeof(BatchZReg) * regs.size(), cudaMemcpyHostToDevice));
 
+    const size_t param_bytes = sizeof(double) * std::max<size_t>(params_.size(), 1);
+    QCSB_CUDA(cudaMalloc(&params_dev_, param_bytes));
+    QCSB_CUDA(cudaMallocHost(&params_host_, param_bytes));
+    upload_params();
+
     // plans: tuned per group, then the final entry layout
     for (Group &g : groups_)
         plan_group(g, clamp_local_bits(kDefaultLocal, g.n));
@@ -635,6 +666,7 @@ void Batch::build()
     tune();
     layout_entries();
     ensure_tensor_mats();
+    upload_recipes();
     fill_entries();
 
     // capture the run: a graph per group, then the results (after dropping
@@ -681,21 +713,14 @@ void Batch::run()
 {
     if (!built_)
         build();
-    // new parameters: each group's entries are filled on the host while the
-    // GPU runs the groups launched before it (the copies of a group read only
-    // its own part of the pinned entry buffer)
-    const bool fill = dirty_;
-    for (size_t gi = 0; gi < groups_.size(); ++gi)
+    QCSB_CUDA(cudaEventRecord(ev0_, stream_));
+    if (dirty_)
     {
-        if (fill)
-            fill_entries((int)gi);
-        if (gi == 0)
-            QCSB_CUDA(cudaEventRecord(ev0_, stream_));
-        QCSB_CUDA(cudaGraphLaunch(execs_[gi], stream_));
+        upload_params();
+        fill_entries();
     }
-    if (groups_.empty())
-        QCSB_CUDA(cudaEventRecord(ev0_, stream_));
-    QCSB_CUDA(cudaGraphLaunch(execs_.back(), stream_));
+    for (cudaGraphExec_t e : execs_)
+        QCSB_CUDA(cudaGraphLaunch(e, stream_));
     dirty_ = false;
     QCSB_CUDA(cudaEventRecord(ev1_, stream_));
     QCSB_CUDA(cudaStreamSynchronize(stream_));
@@ -744,7 +769,7 @@ void Batch::info(qcs_b200_batch_info *out) const
 {
     std::memset(out, 0, sizeof(*out));
     out->circuits = (uint32_t)circuits_.size();
-    out->parameters = num_params_;
+    out->parameters = params_.size();
     uint64_t amps = 0;
     for (const Circuit &c : circuits_)
         amps += 1ull << c.n;

@@ -30,6 +30,42 @@ struct BatchZReg
 constexpr int kBatchZSliceBits = 16;
 constexpr int kBatchZPartials = 17;   // total, 8 sums of the thread bits, 8 of the loop bits
 
+// Gate entries of a batch, evaluated on the GPU from the registers' gate
+// parameters. A recipe says for every entry of a register's block (the same
+// for all registers of a group) which matrix element of which formula it is:
+// element row * 4 + col at the parameters from `index` on, or constant
+// `index` for gates without parameters.
+enum BatchFormula : uint8_t
+{
+    B_CONST, B_GLOBAL_PHASE, B_RX, B_RY, B_RZ, B_P, B_U2, B_U3, B_U4, B_R, B_RXX, B_RYY, B_RZZ, B_RZX, B_XX_PLUS_YY,
+    B_XX_MINUS_YY,
+};
+struct BatchEntry
+{
+    uint8_t formula;
+    uint8_t element;
+    uint16_t pad;
+    uint32_t index;
+};
+static_assert(sizeof(BatchEntry) == 8, "BatchEntry layout");
+
+// Per register, groups one after another and registers in slot order: its
+// block of the entry buffer, its parameters, its group's recipe.
+struct BatchFillReg
+{
+    uint64_t block;
+    uint64_t params;
+    uint32_t recipe, count;
+    uint32_t consts;        // first constant of the group
+    uint32_t pad;
+};
+
+// Fill the entry blocks of registers [0, num_regs) (float2 entries in the
+// first half of a block for complex64).
+template <typename R>
+int launch_batch_fill(const BatchFillReg *regs, uint32_t num_regs, const BatchEntry *recipes, const double2 *consts,
+                      const double *params, double2 *entries, cudaStream_t stream);
+
 template <typename R>
 int launch_batch_zsums(const void *arena, const BatchZItem *items, uint32_t num_items, const BatchZReg *regs,
                        uint32_t num_regs, double *partials, double *out, cudaStream_t stream);
@@ -61,7 +97,6 @@ class Batch
         char name[16];
         int id;      // gate table index (looked up once, at add_circuit)
         int np;
-        double params[4];
         int tq[kMaxTargets];
         uint64_t cmask, cval;
     };
@@ -72,6 +107,7 @@ class Batch
         int group = -1;
         uint32_t slot = 0;       // position among its group's registers
         uint64_t z_off = 0;      // first expectation of this circuit
+        uint64_t param_off = 0;  // first parameter of this circuit
     };
     struct Pass
     {
@@ -92,6 +128,9 @@ class Batch
         int k = 0;
         std::vector<Pass> passes;
         uint32_t stride = 0;             // gate entries per register
+        std::vector<BatchEntry> recipe;  // what they are
+        std::vector<double2> consts;     // the recipe's constants
+        uint32_t first_reg = 0;          // of the group's registers in the fill list
         uint64_t mats_off = 0;           // first entry of the group's registers
         uint64_t amp_off = 0;            // first amplitude of the group's registers
     };
@@ -101,8 +140,10 @@ class Batch
     void plan_group(Group &g, int k, bool tensor = false);
     void ensure_tensor_mats();
     void layout_entries();
-    void fill_entries(int only_group = -1);
-    void fill_group_range(const Group &g, size_t first, size_t last);
+    void make_recipe(Group &g);
+    void upload_recipes();
+    void upload_params();
+    int fill_entries(int only_group = -1);
     void enqueue_passes(const Group &g, cudaStream_t s, int *launches);
     void enqueue_group(int gi, cudaStream_t s, int *launches);
     void enqueue_results(cudaStream_t s, int *launches);
@@ -113,22 +154,26 @@ class Batch
     int amp_bytes_;
     std::vector<Circuit> circuits_;
     std::vector<Group> groups_;
-    uint64_t num_params_ = 0;
+    std::vector<double> params_;   // of all circuits, in order
     bool built_ = false;
     bool ran_ = false;
-    bool dirty_ = false;   // parameters set since the entries were last filled
+    bool dirty_ = false;   // parameters set since the entries were last evaluated
 
     cudaStream_t stream_ = nullptr;
     void *arena_ = nullptr;
     uint64_t total_amps_ = 0;
-    double2 *mats_dev_ = nullptr, *mats_host_ = nullptr;
+    double2 *mats_dev_ = nullptr;
+    double *params_dev_ = nullptr, *params_host_ = nullptr;
+    BatchFillReg *fill_regs_dev_ = nullptr;
+    BatchEntry *recipes_dev_ = nullptr;
+    double2 *consts_dev_ = nullptr;
     uint64_t mats_count_ = 0;
     BatchZItem *zitems_dev_ = nullptr;
     BatchZReg *zregs_dev_ = nullptr;
     uint32_t num_zitems_ = 0;
     double *zpartials_dev_ = nullptr, *zout_dev_ = nullptr, *zout_host_ = nullptr;
     uint64_t zout_count_ = 0;
-    // one graph per group (its entries in, its passes) and one for the
+    // one graph per group (its passes) and one for the
     // results (<Z> of every register, out to the host)
     std::vector<cudaGraphExec_t> execs_;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;

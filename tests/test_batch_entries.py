@@ -1,0 +1,49 @@
+"""Gate entries of a batch, evaluated on the GPU: every parametrised gate of
+at most two targets, with and without controls, before and after
+set_parameters, against the CPU oracle."""
+
+import numpy as np
+import pytest
+
+import qcs_b200
+from qcs_b200 import GATES
+
+pytestmark = pytest.mark.gpu
+N = 10
+
+
+def circuit(rng, names):
+    """h on every qubit, then each gate on random qubits, half of them controlled."""
+    circ = [("h", (), (q,), (), ()) for q in range(N)]
+    for i, name in enumerate(names):
+        npar, nt = GATES[name]
+        qs = [int(q) for q in rng.permutation(N)]
+        ctrls, neg = ((qs[nt],), (qs[nt + 1],)) if i % 2 else ((), ())
+        circ.append((name, tuple(rng.uniform(-7.0, 7.0, npar)), tuple(qs[:nt]), neg, ctrls))
+    return circ
+
+
+@pytest.mark.parametrize("precision", [128, 64])
+@pytest.mark.parametrize("name", [g for g, (npar, nt) in GATES.items() if npar > 0 and nt <= 2] + ["mixed"])
+def test_batch_entries_match_oracle(gpu_lib, oracle_lib, name, precision):
+    """Tolerance: an entry is a product of at most three sines and cosines,
+    each within 2 ulp, over at most 20 gates: 1e-12 holds for complex128;
+    complex64 entries are rounded once to FP32 (6e-8 each): 5e-6."""
+    rng = np.random.default_rng(len(name))
+    names = [name] * 6 if name != "mixed" else [g for g, (_, nt) in GATES.items() if nt <= 2]
+    circ = circuit(rng, names)
+    new = [(op, tuple(rng.uniform(-7.0, 7.0, len(p))), t, neg, pos) for op, p, t, neg, pos in circ]
+    with qcs_b200.Batch(gpu_lib, precision) as batch:
+        for _ in range(3):
+            batch.add_circuit(N, circ)
+        batch.run()
+        first = batch.statevector(2)
+        params = [x for op in circ for x in op[1]]
+        batch.set_parameters(params * 2 + [x for op in new for x in op[1]])
+        batch.run()
+        states = [first, batch.statevector(0), batch.statevector(2)]
+    tol = 1e-12 if precision == 128 else 5e-6
+    for got, ops in zip(states, (circ, circ, new)):
+        with qcs_b200.Simulator(oracle_lib, N) as sim:
+            sim.run(ops)
+            assert np.max(np.abs(got - sim.statevector())) <= tol
