@@ -472,7 +472,7 @@ void Batch::enqueue_passes(const Group &g, cudaStream_t s, int *launches)
             tb.out = static_cast<double2 *>(tmats_dev_);
             tb.regs = static_cast<uint32_t>(g.members.size());
             tb.batch_float = amp_bytes_ == 8 ? 1 : 0;
-            *launches += launch_stage_matrices<double>(prm, tb, s);
+            *launches += launch_stage_matrices(prm, tb, s);
             tp.state = base;
             tp.mats = static_cast<const double2 *>(tmats_dev_);
             tp.reg_mats = tb.nmats;

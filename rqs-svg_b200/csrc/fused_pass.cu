@@ -46,32 +46,170 @@ __global__ void __launch_bounds__(128, sizeof(Real) == 8 ? 3 : 4)
     fused_pass_body<Real, BATCH>(p, [&](const ChunkCtx<V> &cx) { run_stages<V, BATCH>(p, cx); });
 }
 
-// The matrices of a tensor pass: thread (matrix, col) applies the ops of the
-// matrix's stage, exactly as the register stage above applies them, to the
-// unit vector of input slot col, with the stage's condition bits set as the
+// The matrices of a tensor pass: a warp per matrix applies the ops of the
+// matrix's stage to the identity, with the stage's condition bits set as the
 // matrix index says and every other bit outside the stage zero (no op of the
-// stage depends on those). The resulting column M[.][col] is written as the
-// B fragments of the tensor pass's m16n8k8 products, for the real part Mr,
-// the imaginary part Mi and Mr + Mi: B[u][nu] = M[s(nu)][u] for input slot u
-// (tensor layout) and output column nu = 8i + 2t' + e of n-tile i, output
-// slot s(nu) = 8i + t' + 4e; lane 4g + t of fragment 4 * part + 2j + i
-// holds (B[8j + t][8i + g], B[8j + t + 4][8i + g]).
-template <typename Real>
-__global__ void __launch_bounds__(64) stage_matrix_kernel(const __grid_constant__ FPassParams p,
-                                                          const __grid_constant__ TBuildParams tb)
+// stage depends on those). The matrix lives in shared memory, rows in the
+// register stage's slot order, columns in the tensor layout's input slots;
+// the lanes share out (row pair, column) items, an op at a time. It is
+// written as the B fragments of the tensor pass's m16n8k8 products, for the
+// real part Mr, Mi - Mr and -(Mr + Mi): B[u][nu] = M[s(nu)][u] for input slot
+// u (tensor layout) and output column nu = 8i + 2t' + e of n-tile i, output
+// slot s(nu) = 8i + t' + 4e; lane 4g + t of fragment 4 * part + 2j + i holds
+// (B[8j + t][8i + g], B[8j + t + 4][8i + g]).
+// Loops over run-time bits instead of the pass kernel's code unrolled per bit
+// and kind: with a thread per column running that code the build waited on
+// instruction fetches for most of its 17-24 us.
+struct MatrixOps
 {
-    typedef typename Cx<Real>::T V;
-    __shared__ V scratch[64][R];
-    const int width = tb.width;   // 4: 16 x 16 matrices, 3: 8 x 8 (one thread per column)
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t mat = gid >> width;
-    const int col = static_cast<int>(gid & ((1u << width) - 1u));
+    double2 (*m)[R];      // [row][column]
+    int width;            // log2 of the columns
+    uint32_t padmask, padval;   // 8 x 8 stages: the row bit with a fixed value
+
+    // f(row0, row1, column) over the row pairs that differ in bit b
+    template <typename F>
+    __device__ __forceinline__ void pairs(int b, uint32_t cm, uint32_t cv, const F &f) const
+    {
+        for (int i = threadIdx.x & 31; i < (R / 2) << width; i += 32)
+        {
+            const uint32_t h = static_cast<uint32_t>(i) >> width;
+            const uint32_t lo = h & ((1u << b) - 1u);
+            const uint32_t r = lo | ((h ^ lo) << 1);
+            if ((r & cm) == cv && (r & padmask) == padval)
+                f(r, r | (1u << b), i & ((1 << width) - 1));
+        }
+        __syncwarp();
+    }
+    template <typename F>
+    __device__ __forceinline__ void rows(uint32_t cm, uint32_t cv, const F &f) const
+    {
+        for (int i = threadIdx.x & 31; i < R << width; i += 32)
+        {
+            const uint32_t r = static_cast<uint32_t>(i) >> width;
+            if ((r & cm) == cv && (r & padmask) == padval)
+                f(r, m[r][i & ((1 << width) - 1)]);
+        }
+        __syncwarp();
+    }
+    template <typename M>
+    __device__ __forceinline__ void dense1(int b, uint32_t cm, uint32_t cv, const M &ent, int off) const
+    {
+        const double2 e0 = ent[off], e1 = ent[off + 1], e2 = ent[off + 2], e3 = ent[off + 3];
+        pairs(b, cm, cv, [&](uint32_t r0, uint32_t r1, int c) {
+            const double2 x0 = m[r0][c], x1 = m[r1][c];
+            m[r0][c] = cmad2(e0, x0, e1, x1);
+            m[r1][c] = cmad2(e3, x1, e2, x0);
+        });
+    }
+};
+
+// One op other than the runs on a matrix.
+template <typename M>
+__device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, const M &ent, uint32_t j0, uint64_t cbase)
+{
+    const bool tok = (j0 & op.lcmask) == op.lcval && (cbase & op.gcmask) == op.gcval;
+    const uint32_t cm = op.smask, cv = op.sval;
+    if (!tok)
+        return;
+    switch (op.kind)
+    {
+    case F_DENSE1:
+    case F_DENSE1R: w.dense1(op.b0, cm, cv, ent, op.moff); break;
+    case F_DENSE1X4:
+    case F_DENSE1RX4:
+        for (int b = 0; b < kStageBits; ++b)
+            w.dense1(b, 0u, 0u, ent, op.moff + 4 * b);
+        break;
+    case F_DENSE1X2:
+        w.dense1(op.b0, 0u, 0u, ent, op.moff);
+        w.dense1(op.b1, 0u, 0u, ent, op.moff + 4);
+        break;
+    case F_SWAP1:
+        w.pairs(op.b0, cm, cv, [&](uint32_t r0, uint32_t r1, int c) {
+            const double2 t = w.m[r0][c];
+            w.m[r0][c] = w.m[r1][c];
+            w.m[r1][c] = t;
+        });
+        break;
+    case F_DENSE2:
+    case F_SWAP2:
+    {
+        // the condition is written for slot bits in the order b0, b1, then
+        // the other two ascending
+        const uint32_t rest = 15u & ~((1u << op.b0) | (1u << op.b1));
+        const uint32_t c0 = static_cast<uint32_t>(__ffs(rest) - 1), c1 = static_cast<uint32_t>(31 - __clz(rest));
+        for (int i = threadIdx.x & 31; i < (R / 4) << w.width; i += 32)
+        {
+            const uint32_t h = static_cast<uint32_t>(i) >> w.width;
+            const int c = i & ((1 << w.width) - 1);
+            const uint32_t r = ((h & 1u) << c0) | ((h >> 1) << c1);
+            if (((h << 2) & cm) != cv || (r & w.padmask) != w.padval)
+                continue;
+            const uint32_t idx[4] = {r, r | (1u << op.b0), r | (1u << op.b1), r | (1u << op.b0) | (1u << op.b1)};
+            if (op.kind == F_SWAP2)
+            {
+                const double2 t = w.m[idx[1]][c];
+                w.m[idx[1]][c] = w.m[idx[2]][c];
+                w.m[idx[2]][c] = t;
+                continue;
+            }
+            double2 x[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                x[q] = w.m[idx[q]][c];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+            {
+                const int o = op.moff + 4 * q;
+                const double2 y = cmad2(ent[o], x[0], ent[o + 1], x[1]), t = cmad2(ent[o + 2], x[2], ent[o + 3], x[3]);
+                w.m[idx[q]][c] = make_double2(y.x + t.x, y.y + t.y);
+            }
+        }
+        __syncwarp();
+        break;
+    }
+    case F_PHASE:
+    {
+        const double2 e = ent[op.moff];
+        w.rows(cm, cv, [&](uint32_t, double2 &a) { a = cmul(e, a); });
+        break;
+    }
+    case F_MULI:
+        w.rows(cm, cv, [&](uint32_t, double2 &a) { a = op.b1 ? make_double2(a.y, -a.x) : make_double2(-a.y, a.x); });
+        break;
+    default:
+        w.rows(cm, cv, [&](uint32_t r, double2 &a) {
+            uint32_t sub = 0;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (i < op.nt)
+                {
+                    const uint32_t bit = op.spos[i] >= 0   ? r >> op.spos[i]
+                                         : op.loc[i] >= 0 ? j0 >> op.loc[i]
+                                                          : static_cast<uint32_t>(cbase >> op.phys[i]);
+                    sub |= (bit & 1u) << i;
+                }
+            a = cmul(ent[op.moff + sub], a);
+        });
+        break;
+    }
+}
+
+constexpr int kMatrixWarps = 4;   // matrices per block
+
+__global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const __grid_constant__ FPassParams p,
+                                                                         const __grid_constant__ TBuildParams tb)
+{
+    __shared__ double2 scratch[kMatrixWarps][R][R];
+    const int width = tb.width;   // 4: 16 x 16 matrices, 3: 8 x 8
+    const int lane = threadIdx.x & 31;
+    const uint32_t mat = blockIdx.x * kMatrixWarps + threadIdx.x / 32;
     if (mat >= tb.nmats)
         return;
     // batched passes: register reg0 + blockIdx.y, its entries and its matrices
     const uint32_t breg = tb.reg0 + blockIdx.y;
     const void *blk = tb.regs > 0 ? static_cast<const void *>(p.mats + static_cast<size_t>(breg) * p.mat_stride) : nullptr;
-    const BuildEntries<V> ent{p, blk, tb.batch_float, 0u};
+    const BuildEntries<double2> ent{p, blk, tb.batch_float, 0u};
     const uint32_t omat = tb.regs > 0 ? breg * tb.nmats + mat : mat;   // matrix slot written
     int st = 0;
     while (st + 1 < tb.nstages && tb.stages[st + 1].woff <= mat)
@@ -84,46 +222,32 @@ __global__ void __launch_bounds__(64) stage_matrix_kernel(const __grid_constant_
     for (int i = 0; i < S.nlc; ++i)
         if ((v >> i) & 1)
             j0 |= 1u << S.gpos[kStageBits + i];
-    uint64_t local = 0;
-    for (int i = 0; i < k; ++i)
-        local |= p.qbit[i];
-    uint64_t cbase = 0, chunk = 0;
+    uint64_t cbase = 0;
     for (int i = 0; i < S.ngc; ++i)
         if ((v >> (S.nlc + i)) & 1)
-        {
-            const int q = S.gq[i];
-            cbase |= 1ull << q;
-            chunk |= 1ull << (q - __popcll(local & ((1ull << q) - 1)));
-        }
-    // the register pass's thread index of this group: j0 without the stage bits
-    uint32_t tidx = 0;
-    for (int l = 0, pos = 0; l < k; ++l)
-    {
-        if (l == FS.sbits[0] || l == FS.sbits[1] || l == FS.sbits[2] || l == FS.sbits[3])
-            continue;
-        if ((j0 >> l) & 1)
-            tidx |= 1u << pos;
-        ++pos;
-    }
-    // slot u of the tensor layout is slot reg(u) of the register layout; for
-    // 8 x 8 stages the fourth register bit takes the value this matrix's
-    // condition bits give it (it is a group bit of the tensor layout)
-    const int pad = width == 3 && ((j0 >> S.sbits[3]) & 1) ? 1 << ((S.perm >> 6) & 3) : 0;
+            cbase |= 1ull << S.gq[i];
+    // slot u of the tensor layout is row reg(u); for 8 x 8 stages the fourth
+    // register bit takes the value this matrix's condition bits give it (it
+    // is a group bit of the tensor layout)
+    const uint32_t padmask = width == 3 ? 1u << ((S.perm >> 6) & 3) : 0u;
+    const uint32_t padval = (j0 >> S.sbits[3]) & 1u ? padmask : 0u;
+    const uint32_t perm = S.perm;
     auto reg = [&](int u) {
-        int r = pad;
+        uint32_t r = padval;
 #pragma unroll
         for (int b = 0; b < kStageBits; ++b)
             if (b < width && ((u >> b) & 1))
-                r |= 1 << ((S.perm >> (2 * b)) & 3);
+                r |= 1u << ((perm >> (2 * b)) & 3);
         return r;
     };
-    const int r0 = reg(col);
-    V a[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-        a[r] = r == r0 ? V{1, 0} : V{0, 0};
-    const StageSlots<V> ss{scratch[threadIdx.x], 0u, {1u, 2u, 4u, 8u}};
-    const int T = 1 << (k - kStageBits);
+    double2(*m)[R] = scratch[threadIdx.x / 32];
+    for (int i = lane; i < R << width; i += 32)
+        m[i >> width][i & ((1 << width) - 1)] = make_double2(0.0, 0.0);
+    __syncwarp();
+    if (lane < (1 << width))
+        m[reg(lane)][lane] = make_double2(1.0, 0.0);
+    __syncwarp();
+    const MatrixOps w{m, width, padmask, padval};
     for (int oi = FS.op_begin; oi < FS.op_end; ++oi)
     {
         const FOp &op = p.ops[oi];
@@ -132,150 +256,122 @@ __global__ void __launch_bounds__(64) stage_matrix_kernel(const __grid_constant_
             uint32_t neg = 0;
             const int nt = static_cast<int>(op.lcmask);
             for (int i = 1; i <= nt; ++i)
-            {
-                const FOp &t = p.ops[oi + i];
-                if ((j0 & t.lcmask) == t.lcval && (cbase & t.gcmask) == t.gcval)
-                    neg ^= t.moff;
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-            {
-                const uint32_t sgn = ((neg >> r) & 1u) << 31;
-                a[r].x = flip_by(a[r].x, sgn);
-                a[r].y = flip_by(a[r].y, sgn);
-            }
+                neg = sign_term(neg, p.ops[oi + i], j0, cbase);
+            w.rows(0u, 0u, [&](uint32_t r, double2 &a) {
+                if ((neg >> r) & 1)
+                    a = make_double2(-a.x, -a.y);
+            });
             oi += nt;
             continue;
         }
         if (op.kind == F_PRUN)
         {
-            phase_inline<V>(a, op, p.ops + oi + 1, j0, cbase, chunk, static_cast<int>(tidx), T, p.tables,
-                            [&](int off) { return ent[off]; });
-            oi += op.lcmask;
+            // the chunk index and the register pass's thread index of this
+            // matrix's bits, for the run's tables
+            uint64_t local = 0, chunk = 0;
+            for (int i = 0; i < k; ++i)
+                local |= p.qbit[i];
+            for (uint64_t c = cbase; c; c &= c - 1)
+            {
+                const int q = __ffsll(static_cast<long long>(c)) - 1;
+                chunk |= 1ull << (q - __popcll(local & ((1ull << q) - 1)));
+            }
+            uint32_t tidx = 0;
+            for (int l = 0, pos = 0; l < k; ++l)
+            {
+                if (l == FS.sbits[0] || l == FS.sbits[1] || l == FS.sbits[2] || l == FS.sbits[3])
+                    continue;
+                if ((j0 >> l) & 1)
+                    tidx |= 1u << pos;
+                ++pos;
+            }
+            double2 E[kStageBits + 1];
+            phase_tables<double2>(E, op, chunk, static_cast<int>(tidx), 1 << (k - kStageBits), p.tables);
+            const int nterms = static_cast<int>(op.lcmask);
+            for (int i = 1; i <= nterms; ++i)
+                phase_term<double2>(E, p.ops[oi + i], j0, cbase, [&](int off) { return ent[off]; });
+            w.rows(0u, 0u, [&](uint32_t r, double2 &a) {
+                if (op.b1)
+                    a = cmul(ent[op.moff + r], a);
+                if (op.b0 & 1)
+                    a = cmul(E[0], a);
+#pragma unroll
+                for (int b = 0; b < kStageBits; ++b)
+                    if (((op.b0 >> (1 + b)) & 1) && ((r >> b) & 1))
+                        a = cmul(E[1 + b], a);
+            });
+            oi += nterms;
             continue;
         }
-        if ((cbase & op.gcmask) != op.gcval)
-            continue;
-        apply_op<V>(a, op, BuildEntries<V>{p, blk, tb.batch_float, op.moff}, j0, cbase, ss);
+        matrix_op(w, op, ent, j0, cbase);
     }
+    // TF32 high part and the TF32 rounding of the remainder
+    auto split = [](double x, uint32_t &hi, uint32_t &lo) {
+        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(static_cast<float>(x)));
+        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(static_cast<float>(x - __uint_as_float(hi))));
+    };
     if (tb.umma)
     {
         // the 32 x 32 real operand W of a tcgen05 pass (outputs n: Re 0-15,
         // Im 16-31; inputs k likewise): column u of M gives
         // W[u][o] = Mr[o][u], W[u][16 + o] = Mi[o][u],
-        // W[16 + u][o] = -Mi[o][u], W[16 + u][16 + o] = Mr[o][u]; each as a
-        // TF32 high part and the TF32 rounding of the remainder
+        // W[16 + u][o] = -Mi[o][u], W[16 + u][16 + o] = Mr[o][u]
         unsigned char *hi_base = reinterpret_cast<unsigned char *>(tb.out) + static_cast<size_t>(mat) * kUmmaSlab;
         unsigned char *lo_base = hi_base + static_cast<size_t>(tb.nmats) * kUmmaSlab;
-        auto put = [&](int nn, int kk, double w) {
+        auto put = [&](int nn, int kk, double x) {
             const size_t off = static_cast<size_t>((nn >> 3) * 1024 + (kk >> 3) * 256 + ((kk >> 2) & 1) * 128 +
                                                    (nn & 7) * 16 + (kk & 3) * 4);
             uint32_t h, l;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(static_cast<float>(w)));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(static_cast<float>(w - __uint_as_float(h))));
+            split(x, h, l);
             *reinterpret_cast<uint32_t *>(hi_base + off) = h;
             *reinterpret_cast<uint32_t *>(lo_base + off) = l;
         };
-#pragma unroll
-        for (int o = 0; o < R; ++o)
+        for (int i = lane; i < R * R; i += 32)
         {
-            const V y = a[reg(o)];
-            put(o, col, y.x);
-            put(16 + o, col, y.y);
-            put(o, 16 + col, -y.y);
-            put(16 + o, 16 + col, y.x);
+            const int o = i >> 4, u = i & 15;
+            const double2 y = m[reg(o)][u];
+            put(o, u, y.x);
+            put(16 + o, u, y.y);
+            put(o, 16 + u, -y.y);
+            put(16 + o, 16 + u, y.x);
         }
         return;
     }
-    if (width == 3)
-    {
-        // B[u][nu] = M[s(nu)][u], output slot s(nu) = (nu >> 1) + 4 (nu & 1);
-        // lane 4 nu + t of fragment part holds (B[t][nu], B[t + 4][nu])
-        const int b = col >> 2, t = col & 3;
-#pragma unroll
-        for (int nu = 0; nu < 8; ++nu)
+    // fragment (part, j, i) of lane 4g + t: (B[8j + t][8i + g], B[8j + t + 4][8i + g])
+    const int tiles = width == 3 ? 1 : 2;
+    const int g = lane >> 2, t = lane & 3;
+    for (int j = 0; j < tiles; ++j)
+        for (int i = 0; i < tiles; ++i)
         {
-            const V y = a[reg((nu >> 1) + 4 * (nu & 1))];
-            const double parts[3] = {y.x, y.y - y.x, -(y.x + y.y)};
-            const int lane = nu * 4 + t;
+            const uint32_t row = reg(8 * i + (g >> 1) + 4 * (g & 1));
+            const double2 y0 = m[row][8 * j + t], y1 = m[row][8 * j + t + 4];
+            const double parts[3][2] = {{y0.x, y1.x}, {y0.y - y0.x, y1.y - y1.x}, {-(y0.x + y0.y), -(y1.x + y1.y)}};
 #pragma unroll
             for (int part = 0; part < 3; ++part)
             {
+                const size_t f = (static_cast<size_t>(omat) * (3 * tiles * tiles) + part * tiles * tiles + j * tiles + i) * 32 + lane;
                 if (tb.tf32)
                 {
-                    uint32_t hi, lo;
-                    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(static_cast<float>(parts[part])));
-                    asm("cvt.rna.tf32.f32 %0, %1;"
-                        : "=r"(lo)
-                        : "f"(static_cast<float>(parts[part] - __uint_as_float(hi))));
-                    uint32_t *f = reinterpret_cast<uint32_t *>(tb.out) +
-                                  ((static_cast<size_t>(omat) * kTensor3Fragments + part) * 32 + lane) * 4;
-                    f[b] = hi;
-                    f[2 + b] = lo;
+                    uint4 o;
+                    split(parts[part][0], o.x, o.z);
+                    split(parts[part][1], o.y, o.w);
+                    reinterpret_cast<uint4 *>(tb.out)[f] = o;
                 }
                 else
-                {
-                    Real *f = reinterpret_cast<Real *>(tb.out) +
-                              ((static_cast<size_t>(omat) * kTensor3Fragments + part) * 32 + lane) * 2;
-                    f[b] = parts[part];
-                }
+                    tb.out[f] = make_double2(parts[part][0], parts[part][1]);
             }
-        }
-        return;
-    }
-    const int j = col >> 3, b = (col >> 2) & 1, t = col & 3;
-    if (tb.tf32)
-    {
-        // TF32 high part and the TF32 rounding of the remainder, per entry
-        auto split = [](double v, uint32_t &hi, uint32_t &lo) {
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(static_cast<float>(v)));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(static_cast<float>(v - __uint_as_float(hi))));
-        };
-        uint32_t *out = reinterpret_cast<uint32_t *>(tb.out) + static_cast<size_t>(mat) * kTensorFragments * 128;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-            {
-                const V y = a[reg(8 * i + (g >> 1) + 4 * (g & 1))];
-                const double parts[3] = {y.x, y.y - y.x, -(y.x + y.y)};
-                const int lane = g * 4 + t;
-#pragma unroll
-                for (int part = 0; part < 3; ++part)
-                {
-                    uint32_t hi, lo;
-                    split(parts[part], hi, lo);
-                    uint32_t *f = out + ((part * 4 + j * 2 + i) * 32 + lane) * 4;
-                    f[b] = hi;
-                    f[2 + b] = lo;
-                }
-            }
-        return;
-    }
-    Real *out = reinterpret_cast<Real *>(tb.out) + static_cast<size_t>(mat) * kTensorFragments * 64;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-        {
-            const V y = a[reg(8 * i + (g >> 1) + 4 * (g & 1))];
-            const int lane = g * 4 + t;
-            out[((0 * 4 + j * 2 + i) * 32 + lane) * 2 + b] = y.x;
-            out[((1 * 4 + j * 2 + i) * 32 + lane) * 2 + b] = y.y - y.x;
-            out[((2 * 4 + j * 2 + i) * 32 + lane) * 2 + b] = -(y.x + y.y);
         }
 }
 
 } // namespace
 
-template <typename R>
 int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaStream_t stream)
 {
-    const unsigned threads = 64;
-    const unsigned blocks = static_cast<unsigned>((static_cast<uint64_t>(tb.nmats) * (1u << tb.width) + threads - 1) / threads);
+    const unsigned threads = 32 * kMatrixWarps;
+    const unsigned blocks = (tb.nmats + kMatrixWarps - 1) / kMatrixWarps;
     if (tb.regs == 0)
     {
-        stage_matrix_kernel<R><<<blocks, threads, 0, stream>>>(prm, tb);
+        stage_matrix_kernel<<<blocks, threads, 0, stream>>>(prm, tb);
         QCSB_CUDA(cudaGetLastError());
         return 1;
     }
@@ -288,13 +384,12 @@ int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaSt
     {
         slice.reg0 = r0;
         const dim3 grid(blocks, std::min<uint32_t>(tb.regs - r0, 65535u));
-        stage_matrix_kernel<R><<<grid, threads, 0, stream>>>(prm, slice);
+        stage_matrix_kernel<<<grid, threads, 0, stream>>>(prm, slice);
         QCSB_CUDA(cudaGetLastError());
         ++launches;
     }
     return launches;
 }
-template int launch_stage_matrices<double>(const FPassParams &, const TBuildParams &, cudaStream_t);
 
 // ------------------------------------------------------------ planning
 
@@ -2194,7 +2289,7 @@ int FusedExecutor::launch_plan_step(FlushPlan &plan, long st, void *state, const
         tp.state = state;
         tp.err = err_dev_;
         if (build)
-            launches += launch_stage_matrices<double>(prm, tb, stream_);
+            launches += launch_stage_matrices(prm, tb, stream_);
         if (tp.umma)
             launches += launch_tc_pass(tp, stream_);
         else

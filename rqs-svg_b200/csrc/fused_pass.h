@@ -152,7 +152,6 @@ double register_pass_cost(const FPassParams &prm, int amp_bytes);
 double tensor_pass_cost(const TPassParams &tp, int amp_bytes);
 // Builds the pass's matrices (stage_matrix_kernel) and runs the pass;
 // returns the number of kernels launched.
-template <typename R>
 int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaStream_t stream);
 template <typename R>
 int launch_tensor_pass(const TPassParams &tp, cudaStream_t stream);
