@@ -649,19 +649,20 @@ void schedule_stages(const std::vector<GateOp> &q, const PlannedPass &pp, const 
         while (progress)
         {
             progress = false;
+            // the union of the ops left waiting so far: an op is ready when
+            // it commutes with all of them (commute() on the union)
+            OpClass wait{true, 0, 0};
             for (size_t i = 0; i < m; ++i)
             {
                 if (done[i])
                     continue;
-                bool ready = true;
-                for (size_t j = 0; j < i && ready; ++j)
-                    if (!done[j] && !commute(cls[j], cls[i]))
-                        ready = false;
-                if (!ready)
-                    continue;
                 const uint32_t nb = bits | need[i];
-                if (__builtin_popcount(nb) > pp.stage_width)
+                if (!commute(wait, cls[i]) || __builtin_popcount(nb) > pp.stage_width)
+                {
+                    wait.dense |= cls[i].dense;
+                    wait.diag |= cls[i].diag;
                     continue;
+                }
                 bits = nb;
                 ops.push_back((int)i);
                 done[i] = true;
@@ -1250,42 +1251,45 @@ bool build_params_body(const std::vector<GateOp> &q, const PlannedPass &pp, int 
                                     const cplx m = q[r.qi].mat[r.a];
                                     return make_double2(m.re, r.conj ? -m.im : m.im);
                                 };
-                                for (int e = 0; e <= kStageBits; ++e)
-                                {
-                                    if (!((lmask >> e) & 1))
-                                        continue;
-                                    for (size_t t = 0; t < T; ++t)
+                                // one table per factor: the terms' entries
+                                // multiplied in, in order, where their
+                                // condition matches the index
+                                auto add_table = [&](int place, int e, size_t size, const uint32_t *index,
+                                                     const auto &cond) {
+                                    const size_t at = tables->size();
+                                    tables->resize(at + size, make_double2(1.0, 0.0));
+                                    double2 *v = tables->data() + at;
+                                    for (size_t i = 0; i < recs.size(); ++i)
                                     {
-                                        // local index of thread t's slot 0: zeros at the stage bits
-                                        uint32_t j0 = static_cast<uint32_t>(t);
-                                        for (int sb = 0; sb < kStageBits; ++sb)
-                                        {
-                                            const uint32_t lo = j0 & ((1u << sbits[sb]) - 1u);
-                                            j0 = lo | ((j0 ^ lo) << 1);
-                                        }
-                                        double2 v = make_double2(1.0, 0.0);
-                                        for (size_t i = 0; i < recs.size(); ++i)
-                                            if (where[i] == 0 && factor(recs[i].mono) == e &&
-                                                (j0 & recs[i].lcm) == recs[i].lcv)
-                                                v = cmul_host(entry(recs[i]), v);
-                                        tables->push_back(v);
+                                        if (where[i] != place || factor(recs[i].mono) != e)
+                                            continue;
+                                        const double2 x = entry(recs[i]);
+                                        const std::pair<uint32_t, uint32_t> c = cond(i);
+                                        for (size_t t = 0; t < size; ++t)
+                                            if (((index ? index[t] : static_cast<uint32_t>(t)) & c.first) == c.second)
+                                                v[t] = cmul_host(x, v[t]);
+                                    }
+                                };
+                                // local index of thread t's slot 0: zeros at the stage bits
+                                uint32_t slot0[1 << (kMaxLocal - kStageBits)];
+                                for (size_t t = 0; t < T; ++t)
+                                {
+                                    slot0[t] = static_cast<uint32_t>(t);
+                                    for (int sb = 0; sb < kStageBits; ++sb)
+                                    {
+                                        const uint32_t lo = slot0[t] & ((1u << sbits[sb]) - 1u);
+                                        slot0[t] = lo | ((slot0[t] ^ lo) << 1);
                                     }
                                 }
+                                for (int e = 0; e <= kStageBits; ++e)
+                                    if ((lmask >> e) & 1)
+                                        add_table(0, e, T, slot0,
+                                                  [&](size_t i) { return std::make_pair(recs[i].lcm, recs[i].lcv); });
                                 for (int g = 0; g < kMaxChunkGroups; ++g)
                                     for (int e = 0; e <= kStageBits; ++e)
-                                    {
-                                        if (!((gmask[g] >> e) & 1))
-                                            continue;
-                                        for (uint32_t c = 0; c < (1u << kChunkGroupBits); ++c)
-                                        {
-                                            double2 v = make_double2(1.0, 0.0);
-                                            for (size_t i = 0; i < recs.size(); ++i)
-                                                if (where[i] == 1 + g && factor(recs[i].mono) == e &&
-                                                    (c & ccm[i]) == ccv[i])
-                                                    v = cmul_host(entry(recs[i]), v);
-                                            tables->push_back(v);
-                                        }
-                                    }
+                                        if ((gmask[g] >> e) & 1)
+                                            add_table(1 + g, e, size_t(1) << kChunkGroupBits, nullptr,
+                                                      [&](size_t i) { return std::make_pair(ccm[i], ccv[i]); });
                                 packed = lmask;
                                 for (int g = 0; g < kMaxChunkGroups; ++g)
                                     packed |= static_cast<uint64_t>(gmask[g]) << (kChunkGroupBits * (g + 1));
@@ -2477,6 +2481,9 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
     // all of them have gone to the device in one copy (order is kept).
     std::vector<PlannedPass> pieces;
     std::vector<std::vector<StageCond>> conds;
+    // (a parameter block is 28 KiB: growing the vector by copies cost more
+    // than planning the passes)
+    plan->params.reserve(segs.size() + 4);
     size_t launched = 0;   // steps launched while planning
     int launches = 0;
     auto step_features = [&](long st, PassFeatures &f) -> const PassFeatures * {
