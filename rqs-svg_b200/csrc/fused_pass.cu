@@ -619,31 +619,34 @@ std::vector<Segment> plan_greedy(const std::vector<GateOp> &q, int n, int k, int
     return out;
 }
 
-// Order a pass's ops into stages of at most kStageBits local dense bits:
+// Order a pass's ops into stages of at most stage_width local dense bits:
 // repeatedly open a stage and add every op whose dependencies are met and
-// whose dense targets fit, in queue order, until none fits.
+// whose dense targets fit, in queue order, until none fits. With
+// bound_conditions stages also keep the bits they depend on beside their dense ones within
+// what a tensor pass allows (an op that would add more waits for a later
+// stage), so that one gate with a far condition does not take the whole pass
+// off the tensor cores.
 void schedule_stages(const std::vector<GateOp> &q, const PlannedPass &pp, const int *loc_of,
                      std::vector<std::vector<int>> &stage_ops, std::vector<uint32_t> &stage_bits)
 {
     const size_t m = pp.ops.size();
     std::vector<OpClass> cls(m);
-    std::vector<uint32_t> need(m, 0);
+    std::vector<uint32_t> need(m, 0), support(m, 0);   // local bits: dense, all
     for (size_t i = 0; i < m; ++i)
     {
         cls[i] = classify(q[pp.ops[i]]);
-        uint64_t d = cls[i].dense;
-        while (d)
-        {
-            const int b = __builtin_ctzll(d);
-            need[i] |= 1u << loc_of[b];
-            d &= d - 1;
-        }
+        for (uint64_t d = cls[i].dense; d; d &= d - 1)
+            need[i] |= 1u << loc_of[__builtin_ctzll(d)];
+        support[i] = need[i];
+        for (uint64_t d = cls[i].diag & pp.local; d; d &= d - 1)
+            support[i] |= 1u << loc_of[__builtin_ctzll(d)];
     }
     std::vector<bool> done(m, false);
     size_t left = m;
     while (left > 0)
     {
-        uint32_t bits = 0;
+        uint32_t bits = 0, touch = 0;   // local bits: dense, dense or conditions
+        uint64_t chunk_cond = 0;        // condition qubits outside the pass's local ones
         std::vector<int> ops;
         bool progress = true;
         while (progress)
@@ -656,14 +659,20 @@ void schedule_stages(const std::vector<GateOp> &q, const PlannedPass &pp, const 
             {
                 if (done[i])
                     continue;
-                const uint32_t nb = bits | need[i];
-                if (!commute(wait, cls[i]) || __builtin_popcount(nb) > pp.stage_width)
+                const uint32_t nb = bits | need[i], nt = touch | support[i];
+                const uint64_t nc = chunk_cond | (cls[i].diag & ~pp.local);
+                const int lc = __builtin_popcount(nt & ~nb);
+                const bool conds_fit = !pp.bound_conditions || ops.empty() ||
+                                       (lc <= kTensor3TileBits && lc + __builtin_popcountll(nc) <= kTensorMaxCond);
+                if (!commute(wait, cls[i]) || __builtin_popcount(nb) > pp.stage_width || !conds_fit)
                 {
                     wait.dense |= cls[i].dense;
                     wait.diag |= cls[i].diag;
                     continue;
                 }
                 bits = nb;
+                touch = nt;
+                chunk_cond = nc;
                 ops.push_back((int)i);
                 done[i] = true;
                 --left;
@@ -1614,6 +1623,61 @@ bool build_pieces(const std::vector<GateOp> &q, const PlannedPass &pp, int n, st
            build_pieces(q, b, n, params, srcs, pieces, tables, conds);
 }
 
+namespace
+{
+
+// A pass replanned with three dense bits per stage, as 8 x 8 tensor stages:
+// its pieces are appended to params, pieces and conds. False when a piece has
+// no 8 x 8 form (everything is as it was then).
+bool build_tensor8(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes,
+                   std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                   std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out)
+{
+    PlannedPass p3 = pp;
+    p3.stage_width = 3;
+    // complex64 keeps its stages as they are scheduled for the register
+    // path: bounding them would move passes from FP32 gates to split TF32
+    p3.bound_conditions = amp_bytes == (int)sizeof(double2);
+    const size_t before = params.size(), tables_before = tables ? tables->size() : 0;
+    bool ok = build_pieces(q, p3, n, params, nullptr, &pieces, tables, &conds);
+    out = PassChoice();
+    const size_t count = ok ? params.size() - before : 0;
+    out.tparams.resize(count);
+    out.tbuild.resize(count);
+    for (size_t j = 0; ok && j < count; ++j)
+    {
+        ok = make_tensor_params(params[before + j], conds[before + j], amp_bytes, out.tparams[j], out.tbuild[j], 3);
+        out.cost += ok ? tensor_pass_cost(out.tparams[j], amp_bytes) : 0.0;
+        out.tensor.push_back(static_cast<int>(j));
+    }
+    if (!ok)
+    {
+        params.resize(before);
+        pieces.resize(before);
+        conds.resize(before);
+        if (tables)
+            tables->resize(tables_before);
+    }
+    return ok;
+}
+
+// More multi-qubit phases than gates with dense targets (a QFT): the phases
+// reach too many qubits outside their stages to share a few matrices, and a
+// register pass runs them from tables.
+bool mostly_phases(const std::vector<GateOp> &q, const PlannedPass &pp)
+{
+    size_t dense = 0, phases = 0;
+    for (int oi : pp.ops)
+    {
+        const OpClass c = classify(q[oi]);
+        dense += c.dense != 0;
+        phases += c.dense == 0 && (c.diag & (c.diag - 1)) != 0;
+    }
+    return phases > dense;
+}
+
+} // namespace
+
 // How a planned pass runs: its pieces (built by build_pieces and already
 // appended to params / pieces / conds from index `before` on) on the
 // register path or as 16 x 16 tensor stages, per piece whichever the cost
@@ -1627,10 +1691,11 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
                       size_t before, int engine)
 {
     out = PassChoice();
-    // automatic mode: below tensor_min_qubits a register pass's chunks fit
-    // one wave of CTAs, and a tensor pass's extra launch (the matrix build)
-    // costs more than its stages save
-    if (tensor_mode == 1 && n < tensor_min_qubits(amp_bytes))
+    // automatic mode: below tensor_min_qubits a pass that small_tensor_pass
+    // did not take runs on the register path, as do complex128 passes of
+    // mostly phases
+    if (tensor_mode == 1 &&
+        (n < tensor_min_qubits(amp_bytes) || (amp_bytes == (int)sizeof(double2) && mostly_phases(q, pp))))
         tensor_mode = 0;
     double cost4 = 0.0;
     for (size_t i = before; i < params.size(); ++i)
@@ -1661,41 +1726,45 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
     out.cost = cost4;
     if ((tensor_mode != 1 && tensor_mode != 3) || pp.k != kTensorLocal)
         return;
-    PlannedPass p3 = pp;
-    p3.stage_width = 3;
-    std::vector<FPassParams> params3;
-    std::vector<PlannedPass> pieces3;
-    std::vector<std::vector<StageCond>> conds3;
-    const size_t tables_before = tables ? tables->size() : 0;
-    bool ok = build_pieces(q, p3, n, params3, nullptr, &pieces3, tables, &conds3);
-    std::vector<TPassParams> tp3(ok ? params3.size() : 0);
-    std::vector<TBuildParams> tb3(tp3.size());
-    double cost3 = 0.0;
-    for (size_t j = 0; ok && j < params3.size(); ++j)
+    // the 8 x 8 pieces go behind the others and move down in their place
+    PassChoice choice8;
+    const size_t end4 = params.size(), tables_before = tables ? tables->size() : 0;
+    if (!build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, choice8))
+        return;
+    if (tensor_mode == 1 && choice8.cost >= cost4)
     {
-        ok = make_tensor_params(params3[j], conds3[j], amp_bytes, tp3[j], tb3[j], 3);
-        cost3 += ok ? tensor_pass_cost(tp3[j], amp_bytes) : 0.0;
-    }
-    if (!ok || (tensor_mode == 1 && cost3 >= cost4))
-    {
+        params.resize(end4);
+        pieces.resize(end4);
+        conds.resize(end4);
         if (tables)
             tables->resize(tables_before);
         return;
     }
-    params.resize(before);
-    pieces.resize(before);
-    conds.resize(before);
-    out = PassChoice();
-    out.cost = cost3;
-    for (size_t j = 0; j < params3.size(); ++j)
-    {
-        params.push_back(params3[j]);
-        pieces.push_back(pieces3[j]);
-        conds.push_back(std::move(conds3[j]));
-        out.tparams.push_back(tp3[j]);
-        out.tbuild.push_back(tb3[j]);
-        out.tensor.push_back(static_cast<int>(j));
-    }
+    params.erase(params.begin() + before, params.begin() + end4);
+    pieces.erase(pieces.begin() + before, pieces.begin() + end4);
+    conds.erase(conds.begin() + before, conds.begin() + end4);
+    out = std::move(choice8);
+}
+
+// Complex128 registers below tensor_min_qubits take a pass as 8 x 8 tensor
+// stages from the start, without planning its register form first, when it
+// has at least kSmallTensorOps gates and not mostly multi-qubit phases. Measured on B200, us per
+// flush, register path against 8 x 8 stages: a replayed flush of a 12-layer
+// layered circuit 133 -> 88 at 14 qubits, 185 -> 110 at 17, 231 -> 137 at 19;
+// of an ansatz of depth 4 89 -> 53, 126 -> 86, 172 -> 116. A pass of a few
+// gates stays on the register path: its 7-10 us are less than the launch of
+// its matrix build and its own. (Complex64 keeps its FP32 register path
+// there: its split-TF32 products round more.)
+bool small_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out)
+{
+    if (tensor_mode != 1 || amp_bytes != (int)sizeof(double2) || n >= tensor_min_qubits(amp_bytes) ||
+        pp.k != kTensorLocal || pp.ops.size() < kSmallTensorOps)
+        return false;
+    if (mostly_phases(q, pp))
+        return false;
+    return build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, out);
 }
 
 namespace
@@ -2512,7 +2581,10 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
         }
         std::vector<FPassParams> &params = plan->params;
         const size_t before = params.size();
-        if (!build_pieces(ops, s.pass, n, params, nullptr, &pieces, &plan->tables, &conds))
+        PassChoice choice;
+        const bool small = s.width < 0 && small_tensor_pass(ops, s.pass, n, amp_bytes, tensor_mode_, params, pieces, conds,
+                                                            &plan->tables, choice);
+        if (!small && !build_pieces(ops, s.pass, n, params, nullptr, &pieces, &plan->tables, &conds))
         {
             params.resize(before);
             pieces.resize(before);
@@ -2530,9 +2602,9 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
             tmode = 2;
         else if (s.width == 3 && tensor_mode_ != 0)
             tmode = 3;
-        PassChoice choice;
-        choose_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, before,
-                         tensor_engine_);
+        if (!small)
+            choose_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, before,
+                             tensor_engine_);
         for (size_t i = before; i < params.size(); ++i)
         {
             plan->ks.push_back(pieces[i].k);

@@ -33,14 +33,12 @@ struct StageCond
 // the GPU from the pass's ops (stage_matrix_kernel) and applied to every
 // 16-amplitude group of the stage by warp-level MMAs.
 constexpr int kTensorLocal = 11;       // local qubits of a tensor pass (2^11-amplitude chunks)
-// Automatic mode: smaller registers stay on the register path. Measured on
-// B200 (layered, CZ-layered and matching-CX circuits, complex128, and HEA
-// complex64, device time per flush): tensor passes are 20-36% slower at
-// 16-19 qubits, where the register pass's chunks fit one wave of CTAs and
-// a tensor pass adds the matrix build; 5-7% faster at 20 qubits (16% slower
-// for complex64 HEA), 15-52% faster at 21-23.
+// Automatic mode: from these sizes on every pass is priced on each path;
+// smaller complex64 registers stay on the register path, smaller complex128
+// ones take 8 x 8 stages by the rule of small_tensor_pass.
 constexpr int kTensorMinQubits = 20;      // complex128
 constexpr int kTensorMinQubitsC64 = 21;   // complex64
+constexpr size_t kSmallTensorOps = 24;    // gates from which a pass of a small register runs as tensor stages
 inline int tensor_min_qubits(int amp_bytes) { return amp_bytes == 8 ? kTensorMinQubitsC64 : kTensorMinQubits; }
 // Group bits that number a chunk's tiles (tile = warp + 4 x the warp's own
 // tile index): local condition bits go to the lowest ones, the warp bits,
@@ -147,7 +145,7 @@ bool make_tensor_params(const FPassParams &prm, const std::vector<StageCond> &co
 // condition bits per stage); returns the number of kernels launched.
 int launch_tc_pass(const TPassParams &tp, cudaStream_t stream);
 // Estimated time of a pass on the register path and on the tensor path, in
-// one unit (multiply-adds per amplitude at the register path's FP64 rate).
+// picoseconds per amplitude (complex64: in units of its own).
 double register_pass_cost(const FPassParams &prm, int amp_bytes);
 double tensor_pass_cost(const TPassParams &tp, int amp_bytes);
 // Builds the pass's matrices (stage_matrix_kernel) and runs the pass;
@@ -172,6 +170,9 @@ struct PlannedPass
     // 16 x 16 tensor stages) or 3 (8 x 8 tensor stages; the fourth bit of
     // each register-format stage then carries no dense op)
     int stage_width = kStageBits;
+    // stages keep the bits they depend on within a tensor pass's limits
+    // (kTensor3TileBits local ones, kTensorMaxCond in all)
+    bool bound_conditions = false;
 };
 
 struct Segment
@@ -243,6 +244,9 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
                       size_t before, int engine = 1);
+bool small_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out);
 int clamp_local_bits(int k, int n);
 // Complex64 passes read their entries as float2: round count double2 entries
 // in place into the first half of the same memory.

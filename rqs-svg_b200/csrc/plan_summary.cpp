@@ -91,21 +91,28 @@ void plan_summary(int n, const qcs_b200_gate *gates, uint64_t count, qcs_b200_pl
         std::vector<FPassParams> params;
         std::vector<PlannedPass> pieces;
         std::vector<std::vector<StageCond>> conds;
-        if (!build_pieces(queue, s.pass, n, params, nullptr, &pieces, &tables, &conds))
-        {
-            out.plain_gates += static_cast<uint32_t>(s.pass.ops.size());
-            continue;
-        }
-        for (size_t pi = 0; pi < params.size(); ++pi)
-        {
-            TPassParams tp;
-            TBuildParams tb;
-            if (make_tensor_params(params[pi], conds[pi], 16, tp, tb))
-                ++out.tensor_eligible;
-        }
         // the executor's choice for a complex128 register (automatic mode)
         PassChoice choice;
-        choose_execution(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice, 0);
+        if (small_tensor_pass(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice))
+        {
+            out.tensor_eligible += static_cast<uint32_t>(params.size());
+        }
+        else
+        {
+            if (!build_pieces(queue, s.pass, n, params, nullptr, &pieces, &tables, &conds))
+            {
+                out.plain_gates += static_cast<uint32_t>(s.pass.ops.size());
+                continue;
+            }
+            for (size_t pi = 0; pi < params.size(); ++pi)
+            {
+                TPassParams tp;
+                TBuildParams tb;
+                if (make_tensor_params(params[pi], conds[pi], 16, tp, tb))
+                    ++out.tensor_eligible;
+            }
+            choose_execution(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice, 0);
+        }
         for (size_t pi = 0; pi < params.size(); ++pi)
         {
             const FPassParams &p = params[pi];

@@ -695,12 +695,21 @@ bool make_tensor_params(const FPassParams &prm, const std::vector<StageCond> &co
     return true;
 }
 
-// Pass costs in one unit (multiply-adds per amplitude at the register path's
-// FP64 rate), calibrated on B200 with the 30-qubit layered and matching
-// circuits: register passes keep the FP64 pipe about 45% busy; complex64
-// register passes take about 0.75 of the complex128 time; a complex128
-// 16 x 16 tensor stage measured like 82 units, a complex64 one like 30.
-double register_pass_cost(const FPassParams &prm, int amp_bytes)
+// Pass costs of complex128 in picoseconds per amplitude, fitted on B200 to
+// pass timings at 25 qubits (layered, matching and ansatz circuits and random
+// gates of every kind; 280 to 300 passes per path): 8 x 8 stages 2.8 + 1.55
+// per stage (a random-gate pass of four stages 8.8), 16 x 16 stages 2.0 + 3.1
+// per stage, register passes 18-21 ps on the three families and 24 on random
+// gates, of which the former estimate, multiply-adds alone, saw half: the
+// exchanges, predicated gates and the stages' own loads and stores were
+// missing, and passes of few, mixed gates stayed on the register path.
+// Complex64 keeps the estimate by multiply-adds (8 x 8 stages 28 units, 16 x
+// 16 ones 30, a register pass's FP32 operations over 0.6): its tensor passes
+// round more than its FP32 gates, so a better estimate of their time would
+// move passes to the less exact path.
+namespace
+{
+double register_pass_units_c64(const FPassParams &prm)
 {
     double fma = 0.0;
     for (int o = 0; o < prm.nops; ++o)
@@ -720,23 +729,45 @@ double register_pass_cost(const FPassParams &prm, int amp_bytes)
         default: fma += 0.5; break;   // exchanges, sign flips, terms
         }
     }
-    return fma / 0.45 * (amp_bytes == 8 ? 0.75 : 1.0);
+    return fma / 0.6;
+}
+} // namespace
+
+double register_pass_cost(const FPassParams &prm, int amp_bytes)
+{
+    if (amp_bytes == 8)
+        return register_pass_units_c64(prm);
+    double ps = 1.7 + 1.2 * prm.nstages;
+    for (int o = 0; o < prm.nops; ++o)
+    {
+        const FOp &op = prm.ops[o];
+        const bool predicated = op.smask != 0 || op.lcmask != 0;
+        switch (op.kind)
+        {
+        case F_DENSE1: ps += predicated ? 1.2 : 0.66; break;
+        case F_DENSE1R: ps += predicated ? 0.7 : 0.33; break;
+        case F_DENSE1X4: ps += 2.6; break;
+        case F_DENSE1RX4: ps += 1.3; break;
+        case F_DENSE1X2: ps += 1.3; break;
+        case F_DENSE2: ps += 2.8; break;
+        case F_SWAP2: ps += 1.7; break;
+        case F_PHASE: ps += 0.6; break;
+        case F_DIAG: ps += 0.9; break;
+        case F_PRUN: ps += 0.4 + 0.33 * __builtin_popcount(op.b0) + (op.b1 ? 0.35 : 0.0); break;
+        case F_SIGNS: ps += 0.25; break;
+        case F_SIGNT: ps += 0.05; break;
+        case F_TERM: ps += 0.1; break;
+        default: ps += 0.5; break;   // exchanges, phases by +-i
+        }
+    }
+    return ps;
 }
 
 double tensor_pass_cost(const TPassParams &tp, int amp_bytes)
 {
-    // an 8 x 8 stage: half the tensor-core work of a 16 x 16 one and the
-    // same shared-memory round trip; measured on the 30-qubit layered and
-    // matching circuits: 0.63 of a 16 x 16 stage for complex128, 0.93 for
-    // complex64 (whose stages are not bound by the tensor pipe). complex128
-    // stages lost 10% of their time when the additions after the products
-    // went into the tensor cores' accumulation (the factors below)
-    if (tp.width == 3)
-        return (amp_bytes == 8 ? 28.0 : 47.0) * tp.nstages;
-    // tcgen05 16 x 16 stages (complex64): measured 1% below mma.sync ones
-    if (tp.umma)
-        return 29.0 * tp.nstages;
-    return (amp_bytes == 8 ? 30.0 : 74.0) * tp.nstages;
+    if (amp_bytes == 8)
+        return (tp.width == 3 ? 28.0 : tp.umma ? 29.0 : 30.0) * tp.nstages;   // tcgen05: 1% below mma.sync
+    return tp.width == 3 ? 2.8 + 1.55 * tp.nstages : 2.0 + 3.1 * tp.nstages;
 }
 
 template <typename R>
