@@ -140,3 +140,31 @@ def test_collapse_only_flush(gpu_lib, oracle_lib, precision):
         assert float(np.max(np.abs(got - ref))) <= tol
         # one amplitude is left: the measured basis state
         assert np.count_nonzero(got) == 1
+
+
+@pytest.mark.parametrize("precision", [128, 64])
+@pytest.mark.parametrize("n", [9, 11, 16, 22, 23])
+def test_queues_of_one_or_two_launches(gpu_lib, oracle_lib, n, precision):
+    """Flushes of one to three gates, alone and behind collapses (a chain of
+    them, and one of a qubit that is collapsed again), below and above the
+    size up to which they run gate by gate: clbits and state as the oracle's."""
+    circ = C.layered_u3_cz(n, 2, seed=n)
+    h = ("h", (), (4,), (), ())
+    flushes = [[h], [("u3", (0.3, 0.4, 0.5), (1,), (), (3,)), ("x", (), (0,), (8,), ())],
+               [("x", (), (q,), (), ()) for q in (0, 5, 7)]]
+    measured = [[0], [0, 3, 6], [4], [4, 8, 0]]
+    results = []
+    for lib in (gpu_lib, oracle_lib):
+        kw = {"precision": precision, "fusion": qcs_b200.FUSION_GREEDY} if lib is gpu_lib else {}
+        with qcs_b200.Simulator(lib, n, n, seed=5, **kw) as sim:
+            sim.run(circ)
+            bits = [sim.measure(q) for q in measured[0]]
+            for ops, qs in zip(flushes, measured[1:]):
+                sim.run(ops)
+                bits += [sim.measure(q) for q in qs]
+                sim.reset(qs[0])
+            results.append((bits, sim.statevector()))
+    (bits, state), (ref_bits, ref) = results
+    assert bits == ref_bits
+    # at most 2 layers and 8 gates of FP32 roundings (6e-8 each) for complex64
+    assert np.max(np.abs(state - ref)) <= (1e-12 if precision == 128 else 1e-5)
