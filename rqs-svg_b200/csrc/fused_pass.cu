@@ -2371,6 +2371,13 @@ int FusedExecutor::launch_plan_step(FlushPlan &plan, long st, void *state, const
         stats.tensor8_passes += tp.width == 3 ? 1 : 0;
         stats.tcgen05_passes += tp.umma ? 1 : 0;
     }
+    else if (plan.butterfly_of[st] >= 0)
+    {
+        BPassParams &bp = plan.bparams[plan.butterfly_of[st]];
+        bp.state = state;
+        bp.tables = tables_dev;
+        launches += c64 ? launch_butterfly_pass<float>(bp, stream_) : launch_butterfly_pass<double>(bp, stream_);
+    }
     else
     {
         launches += c64 ? launch_fused_pass<float>(state, plan.ks[st], prm, stream_)
@@ -2653,6 +2660,15 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
                 plan->tensor_of.push_back(-1);
             }
         }
+        // register passes of Hadamard gates and diagonals run as butterflies
+        for (size_t i = before; i < params.size(); ++i)
+        {
+            BPassParams bp;
+            const bool ok = plan->tensor_of[i] < 0 && make_butterfly_params(params[i], amp_bytes, bp);
+            plan->butterfly_of.push_back(ok ? static_cast<int>(plan->bparams.size()) : -1);
+            if (ok)
+                plan->bparams.push_back(bp);
+        }
         // complex64 register passes read their entries as float2; tensor
         // passes build their matrices from the double2 entries
         for (size_t i = before; i < params.size(); ++i)
@@ -2676,7 +2692,8 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
     // plans whose parameter blocks would take much host memory (a flush of
     // thousands of passes) are not kept
     const size_t plan_bytes = plan->params.size() * sizeof(FPassParams) + plan->tparams.size() * sizeof(TPassParams) +
-                              plan->tbuild.size() * sizeof(TBuildParams) + plan->tables.size() * sizeof(double2);
+                              plan->tbuild.size() * sizeof(TBuildParams) + plan->bparams.size() * sizeof(BPassParams) +
+                              plan->tables.size() * sizeof(double2);
     if (!timer.enabled && !timed_flush && plan_bytes <= kKeptPlanBytes)
     {
         plan->queued = queued;

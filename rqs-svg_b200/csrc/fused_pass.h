@@ -154,6 +154,49 @@ int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaSt
 template <typename R>
 int launch_tensor_pass(const TPassParams &tp, cudaStream_t stream);
 
+// Butterfly passes (butterfly_pass.cu): stages of Hadamard gates, highest
+// stage bit first, and diagonal runs. Step b of a stage is bit b's H and the
+// diagonals that follow it, step kStageBits the diagonals before any H.
+constexpr int kButterflyStages = 8;
+constexpr int kButterflyEntries = 256;
+struct BRun
+{
+    uint64_t packed;   // tables as an F_PRUN's: gcmask, lcval, b0
+    uint32_t table;
+    uint32_t used;
+};
+struct BStep
+{
+    uint8_t h;
+    uint8_t factors;   // 0 none, 1 one per slot with the step's bit, 2 one per slot
+    uint16_t entry;
+    uint32_t pad;
+    BRun run;
+};
+struct BStage
+{
+    uint8_t sbits[kStageBits];
+    uint8_t pad[4];
+    BStep steps[kStageBits + 1];
+};
+struct BPassParams
+{
+    void *state;
+    const double2 *tables;
+    uint64_t chunks;
+    uint64_t qmasks[kMaxLocal];
+    uint64_t qbit[kMaxLocal];
+    double scale;              // 2^(-m/2) for the pass's m Hs
+    int nstages;
+    int direct_in, direct_out; // the first / last stage leaves local bits 0..2 alone
+    BStage stages[kButterflyStages];
+    double2 entries[kButterflyEntries];   // complex64: float2 entries in the first half
+};
+// False when the pass (entries as double2) has any other gate.
+bool make_butterfly_params(const FPassParams &prm, int amp_bytes, BPassParams &bp);
+template <typename R>
+int launch_butterfly_pass(const BPassParams &bp, cudaStream_t stream);
+
 struct OpClass
 {
     bool fusable;

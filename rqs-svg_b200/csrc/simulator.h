@@ -270,6 +270,8 @@ class FusedExecutor
         std::vector<int> tensor_of;   // per pass: index into tparams / tbuild, or -1
         std::vector<TPassParams> tparams;
         std::vector<TBuildParams> tbuild;
+        std::vector<int> butterfly_of;   // per pass: index into bparams, or -1
+        std::vector<BPassParams> bparams;
         std::vector<long> steps;      // launch order: >= 0 a pass, < 0 plain op -1 - step
         std::vector<double2> tables;  // phase-run tables of the passes
         // The tensor passes' stage matrices, kept on the device from the
