@@ -51,12 +51,10 @@ namespace
 {
 
 constexpr int kThreads = 1 << (kTensorLocal - kStageBits);   // 128: 4 warps, two 16-group tiles each
-// chunk buffers of a tensor pass's CTA: 2 (double-buffered: the next chunk
-// streams in during this one's stages; three CTAs per SM) or 1 (more CTAs
-// per SM instead: four for 16 x 16 stages at 128 registers, measured 5.5-5.8%
-// faster on the 30-qubit circuits; six or eight for 8 x 8 stages, below)
-constexpr int kTensor3Buffers = 1;
-constexpr int kTensor4Buffers = 1;
+// One chunk buffer per CTA and more CTAs per SM, instead of two buffers (the
+// next chunk streaming in during this one's stages) and three CTAs: four for
+// 16 x 16 stages at 128 registers measured 5.5-5.8% faster on the 30-qubit
+// circuits.
 constexpr int kSlots = 1 << kStageBits;
 constexpr int kChunk = 1 << kTensorLocal;
 
@@ -161,8 +159,8 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 template <typename Real>
 constexpr int tensor_ctas_per_sm() { return sizeof(Real) == 8 ? 5 : 5; }
 
-template <typename Real, int NBUF>
-__global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor_ctas_per_sm<Real>() : 3) tensor_pass_kernel(const __grid_constant__ TPassParams p)
+template <typename Real>
+__global__ void __launch_bounds__(kThreads, tensor_ctas_per_sm<Real>()) tensor_pass_kernel(const __grid_constant__ TPassParams p)
 {
     typedef Tensor<Real> TT;
     typedef typename TT::V V;
@@ -240,24 +238,15 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor_ctas_per_sm<Real>
         return;
     uint64_t cbase_next = chunk_base(c);
     issue_load(cbase_next, smem);
-    int cur = 0;
     for (; c < p.chunks; c += gridDim.x)
     {
-        // NBUF as in tensor3_pass_kernel
-        V *sb = smem + (NBUF == 2 ? cur * kChunk : 0);
+        // one chunk buffer, as in tensor3_pass_kernel
+        V *sb = smem;
         const uint64_t cbase = cbase_next;
         const uint64_t next = c + gridDim.x;
         if (next < p.chunks)
             cbase_next = chunk_base(next);
-        if (NBUF == 2 && next < p.chunks)
-        {
-            issue_load(cbase_next, smem + (cur ^ 1) * kChunk);
-            cp_wait<1>();
-        }
-        else
-        {
-            cp_wait<0>();
-        }
+        cp_wait<0>();
         __syncthreads();
 
         for (int st = 0; st < p.nstages; ++st)
@@ -327,10 +316,24 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor_ctas_per_sm<Real>
         for (int m = 0; m < kSlots; ++m)
             __stcs(state + (cbase | elem_offset(m)), sb[TT::swz(tid + m * kThreads)]);
         __syncthreads();
-        if (NBUF == 1 && next < p.chunks)
+        if (next < p.chunks)
             issue_load(cbase_next, smem);
-        cur ^= 1;
     }
+}
+
+// A stage's shared-memory offsets (TPassParams::swz), read a stage ahead: a
+// first read of parameter memory takes longer than a tile's products.
+struct StageLayout
+{
+    uint32_t w[6];
+};
+__device__ __forceinline__ StageLayout stage_layout(const TPassParams &p, int st)
+{
+    StageLayout l;
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        l.w[i] = reinterpret_cast<const uint32_t *>(p.swz[st])[i];
+    return l;
 }
 
 // 8 x 8 stages (three slot bits; TPassParams::width 3). A warp takes 16
@@ -339,27 +342,40 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor_ctas_per_sm<Real>
 // single n-tile stands for output slot t + 4e, so the lane stores to the
 // positions it loaded. Three m16n8k8 products per 16 rows (as above):
 // 24 multiply-adds per amplitude and stage, half those of a 16 x 16 stage
-// for three quarters of its qubits. 256 rows per chunk: 16 tiles, four per
-// warp; group bits 4..7 pick the tile, warp + 4 x the warp's tile index (the
-// stage's local condition bits are the lowest group bits, so with at most
-// two of them a warp runs all its tiles with one matrix, fetched before the
-// stage begins).
-// CTAs per SM of the single-buffered 8 x 8 pass: six for complex128 (80
-// registers; 6 x 32 KiB of chunk), eight for complex64 (64 registers); each
-// step from four measured faster (30-qubit layered and matching complex128:
-// 0.6998 -> 0.6725 -> 0.6551 s and 1.2803 -> 1.2310 -> 1.1979 s at 4, 5, 6)
-template <typename Real>
-constexpr int tensor3_ctas_per_sm() { return sizeof(Real) == 8 ? 6 : 8; }
+// for three quarters of its qubits. 256 rows per chunk: 16 tiles over the W
+// warps of a CTA; group bits 4..7 pick the tile, warp + W x the warp's tile
+// index (the stage's local condition bits are the lowest group bits, so with
+// at most log2 W of them a warp runs all its tiles with one matrix, fetched
+// before the stage begins).
+// W = 4: six CTAs per SM for complex128 (80 registers; 6 x 32 KiB of chunk),
+// eight for complex64 (64 registers); each step from four measured faster
+// (30-qubit layered and matching complex128: 0.6998 -> 0.6725 -> 0.6551 s and
+// 1.2803 -> 1.2310 -> 1.1979 s at 4, 5, 6). That needs as many chunks: a
+// register with few leaves a warp to work through four tiles one after another
+// on a nearly idle SM. W = 8 (two tiles per warp) up to 256 chunks: layered
+// circuit 117 -> 106 us at 17 qubits, 143 -> 135 at 19, but 195 -> 214 at 20,
+// 542 -> 612 at 22; 16 warps measured like 8 and worse from 19 qubits on.
+// complex128: the stage layouts are read one stage ahead (the 30-qubit step
+// 594 -> 590 ms) and the last stage stores its outputs straight to the
+// register instead of through shared memory (590 -> 576 ms; 21 qubits 336 ->
+// 319 us); with low qubits off the lanes that measured 3% slower, and
+// complex64, whose 64-byte runs it halves, lost 1%.
+template <typename Real, int W>
+constexpr int tensor3_ctas_per_sm() { return W == 4 ? (sizeof(Real) == 8 ? 6 : 8) : 4; }
 
-template <typename Real, int NBUF>
-__global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real>() : 3)
+template <typename Real, int W>
+__global__ void __launch_bounds__(32 * W, tensor3_ctas_per_sm<Real, W>())
     tensor3_pass_kernel(const __grid_constant__ TPassParams p)
 {
     typedef Tensor<Real> TT;
     typedef typename TT::V V;
     typedef typename TT::Frag Frag;
+    constexpr int kT = 32 * W;                       // threads
+    constexpr int kWarpBits = W == 4 ? 2 : 3;
+    constexpr int kElemBits = kTensorLocal - 5 - kWarpBits;   // amplitudes per thread of a chunk's copy: 2^kElemBits
+    constexpr int kTiles = 16 / W;                   // tiles per warp
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V *smem = reinterpret_cast<V *>(smem_raw);
+    V *sb = reinterpret_cast<V *>(smem_raw);
     V *const state = static_cast<V *>(p.state);
     const Frag *const mats = reinterpret_cast<const Frag *>(p.mats);
     const int tid = threadIdx.x;
@@ -367,13 +383,13 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
     const int g = lane >> 2, t = lane & 3;
 
     uint64_t dep_tid = 0;
-    for (int i = 0; i < kTensorLocal - kStageBits; ++i)
+    for (int i = 0; i < kTensorLocal - kElemBits; ++i)
         if ((tid >> i) & 1)
             dep_tid |= p.qbit[i];
-    uint64_t hb[kStageBits];
+    uint64_t hb[kElemBits];
 #pragma unroll
-    for (int b = 0; b < kStageBits; ++b)
-        hb[b] = p.qbit[kTensorLocal - kStageBits + b];
+    for (int b = 0; b < kElemBits; ++b)
+        hb[b] = p.qbit[kTensorLocal - kElemBits + b];
     // batched passes: the register's amplitudes start at register << n (the
     // bits above n of the base; matrix choices read bits below n only)
     auto chunk_base = [&](uint64_t c) -> uint64_t {
@@ -390,26 +406,26 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
     auto elem_offset = [&](int m) -> uint64_t {
         uint64_t off = dep_tid;
 #pragma unroll
-        for (int b = 0; b < kStageBits; ++b)
+        for (int b = 0; b < kElemBits; ++b)
             if ((m >> b) & 1)
                 off |= hb[b];
         return off;
     };
-    auto issue_load = [&](uint64_t cb, V *dst) {
+    auto issue_load = [&](uint64_t cb) {
         if (p.from_zero)
         {
 #pragma unroll
-            for (int m = 0; m < kSlots; ++m)
+            for (int m = 0; m < (1 << kElemBits); ++m)
             {
                 const bool one = (cb & ((1ull << p.n) - 1)) == 0 && m == 0 && tid == 0;
-                dst[TT::swz(tid + m * kThreads)] = V{one ? Real(1) : Real(0), Real(0)};
+                sb[TT::swz(tid + m * kT)] = V{one ? Real(1) : Real(0), Real(0)};
             }
         }
         else
         {
 #pragma unroll
-            for (int m = 0; m < kSlots; ++m)
-                TT::cp_async(dst + TT::swz(tid + m * kThreads), state + (cb | elem_offset(m)));
+            for (int m = 0; m < (1 << kElemBits); ++m)
+                TT::cp_async(sb + TT::swz(tid + m * kT), state + (cb | elem_offset(m)));
         }
         cp_commit();
     };
@@ -418,13 +434,12 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
     int bf_st = -1;
     uint32_t bf_v = 0;
     uint64_t bf_reg = 0;   // register whose matrices bf holds (batched passes)
-    auto matrix_of = [&](int st, uint64_t cb, int mt) -> uint32_t {
+    auto matrix_of = [&](int st, uint64_t cb) -> uint32_t {
         const TStage &S = p.stages[st];
         uint32_t vc = 0;
         for (int i = 0; i < S.ngc; ++i)
             vc |= static_cast<uint32_t>((cb >> S.gq[i]) & 1) << i;
-        const uint32_t tile = static_cast<uint32_t>(warp | (mt << 2));
-        return (tile & ((1u << S.nlc) - 1u)) | (vc << S.nlc);
+        return (static_cast<uint32_t>(warp) & ((1u << S.nlc) - 1u)) | (vc << S.nlc);
     };
     auto fetch = [&](int st, uint32_t v, uint64_t cb) {
         const uint64_t reg = cb >> p.n;
@@ -438,45 +453,61 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
         bf_reg = reg;
     };
 
+    // complex128: the last stage's outputs go straight to the register, at the
+    // register bits of the lane's and warp's group and slot positions (fixed
+    // for the pass), the upper row and slot bits and the tile bits above the
+    // warp's
+    constexpr bool kDirect = sizeof(Real) == 8;
+    const TStage &out_stage = p.stages[p.nstages - 1];
+    uint64_t out_off = 0;
+    if (kDirect)
+    {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if ((g >> i) & 1)
+                out_off |= p.qbit[out_stage.gpos[i]];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if ((t >> i) & 1)
+                out_off |= p.qbit[out_stage.sbits[i]];
+#pragma unroll
+        for (int i = 0; i < kWarpBits; ++i)
+            if ((warp >> i) & 1)
+                out_off |= p.qbit[out_stage.gpos[4 + i]];
+    }
+
     uint64_t c = blockIdx.x;
     if (c >= p.chunks)
         return;
     uint64_t cbase_next = chunk_base(c);
-    issue_load(cbase_next, smem);
+    issue_load(cbase_next);
+    StageLayout next_layout = stage_layout(p, 0);
     if (p.nstages > 0)
-        fetch(0, matrix_of(0, cbase_next, 0), cbase_next);
-    int cur = 0;
+        fetch(0, matrix_of(0, cbase_next), cbase_next);
     for (; c < p.chunks; c += gridDim.x)
     {
-        // NBUF 2: the next chunk streams in while this one is processed;
-        // NBUF 1: one buffer, loaded after the last one's stores (more CTAs
-        // per SM instead)
-        V *sb = smem + (NBUF == 2 ? cur * kChunk : 0);
+        // one chunk buffer, loaded after the last one's stores: the other
+        // CTAs of the SM work meanwhile
         const uint64_t cbase = cbase_next;
         const uint64_t next = c + gridDim.x;
         if (next < p.chunks)
             cbase_next = chunk_base(next);
-        if (NBUF == 2 && next < p.chunks)
-        {
-            issue_load(cbase_next, smem + (cur ^ 1) * kChunk);
-            cp_wait<1>();
-        }
-        else
-        {
-            cp_wait<0>();
-        }
+        cp_wait<0>();
         __syncthreads();
 
         for (int st = 0; st < p.nstages; ++st)
         {
-            const uint16_t *sw = p.swz[st];
+            // (complex64 has the registers for its CTAs only without it)
+            const StageLayout L = sizeof(Real) == 8 ? next_layout : stage_layout(p, st);
+            if (sizeof(Real) == 8)
+                next_layout = stage_layout(p, st + 1 < p.nstages ? st + 1 : 0);
             uint32_t gbit[8], sbit[3];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                gbit[i] = sw[i];
+                gbit[i] = (L.w[i / 2] >> (16 * (i % 2))) & 0xffffu;
 #pragma unroll
             for (int b = 0; b < 3; ++b)
-                sbit[b] = sw[8 + b];
+                sbit[b] = (L.w[(8 + b) / 2] >> (16 * (b % 2))) & 0xffffu;
             const uint32_t lane_pos = ((g & 1) ? gbit[0] : 0u) ^ ((g & 2) ? gbit[1] : 0u) ^
                                       ((g & 4) ? gbit[2] : 0u) ^ ((t & 1) ? sbit[0] : 0u) ^ ((t & 2) ? sbit[1] : 0u);
             const uint32_t hpos = gbit[3];
@@ -489,9 +520,9 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
             const uint32_t vlo = (1u << S.nlc) - 1u, vhi = vc << S.nlc;
             const uint64_t creg = cbase >> p.n;
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+            for (int mt = 0; mt < kTiles; ++mt)
             {
-                const uint32_t tile = static_cast<uint32_t>(warp | (mt << 2));
+                const uint32_t tile = static_cast<uint32_t>(warp | (mt << kWarpBits));
                 const uint32_t v = (tile & vlo) | vhi;
                 if (bf_st != st || bf_v != v || bf_reg != creg)
                     fetch(st, v, cbase);
@@ -510,24 +541,41 @@ __global__ void __launch_bounds__(kThreads, NBUF == 1 ? tensor3_ctas_per_sm<Real
                 TT::mma(yr, ai, bf[2]);
                 TT::mma(yi, ar, bf[1]);
                 // e = 0: row g, slot t; 1: row g, slot t + 4; 2, 3: row g + 8
+                if (!kDirect || st + 1 < p.nstages)
+                {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    sb[pos(e >> 1, e & 1)] = V{yr[e], yi[e]};
+                    for (int e = 0; e < 4; ++e)
+                        sb[pos(e >> 1, e & 1)] = V{yr[e], yi[e]};
+                }
+                else
+                {
+                    V *out = state + (cbase | out_off);
+#pragma unroll
+                    for (int i = 0; i < 4 - kWarpBits; ++i)
+                        if ((mt >> i) & 1)
+                            out += p.qbit[out_stage.gpos[4 + kWarpBits + i]];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        __stcs(out + (((e >> 1) ? p.qbit[out_stage.gpos[3]] : 0) + ((e & 1) ? p.qbit[out_stage.sbits[2]] : 0)),
+                               V{yr[e], yi[e]});
+                }
             }
             if (st + 1 < p.nstages)
-                fetch(st + 1, matrix_of(st + 1, cbase, 0), cbase);
+                fetch(st + 1, matrix_of(st + 1, cbase), cbase);
             else if (next < p.chunks)
-                fetch(0, matrix_of(0, cbase_next, 0), cbase_next);
+                fetch(0, matrix_of(0, cbase_next), cbase_next);
             __syncthreads();
         }
 
+        if (!kDirect)
+        {
 #pragma unroll
-        for (int m = 0; m < kSlots; ++m)
-            __stcs(state + (cbase | elem_offset(m)), sb[TT::swz(tid + m * kThreads)]);
-        __syncthreads();
-        if (NBUF == 1 && next < p.chunks)
-            issue_load(cbase_next, smem);
-        cur ^= 1;
+            for (int m = 0; m < (1 << kElemBits); ++m)
+                __stcs(state + (cbase | elem_offset(m)), sb[TT::swz(tid + m * kT)]);
+            __syncthreads();
+        }
+        if (next < p.chunks)
+            issue_load(cbase_next);
     }
 }
 
@@ -612,21 +660,31 @@ bool make_tensor_params(const FPassParams &prm, const std::vector<StageCond> &co
         if (woff + nm > static_cast<uint32_t>(kTensorMaxMats))
             return false;
         TStage &S = tp.stages[s];
-        // slot bits 0 and 1: two of distinct residues where there are
+        // The last stage of a complex128 8 x 8 pass stores its outputs
+        // straight to the register: local positions 0..2 (qubits 0..2, the
+        // contiguous 128-byte runs) then sit on lane bits (slot bits 0 and 1,
+        // group bits 0..2) wherever the stage allows it, so that a warp's
+        // store covers whole runs.
+        const bool direct = width == 3 && !c64 && s + 1 == prm.nstages;
+        // slot bits 0 and 1: two of distinct residues where there are, in a
+        // direct stage the pair with the most low positions
         int order[kStageBits] = {slots[0], slots[1], slots[2], slots[3 % nslots]};
-        bool found = false;
-        for (int a = 0; a < nslots && !found; ++a)
-            for (int b = a + 1; b < nslots && !found; ++b)
-                if (FS.sbits[slots[a]] % mod != FS.sbits[slots[b]] % mod)
-                {
-                    int rest = 0;
-                    order[0] = slots[a];
-                    order[1] = slots[b];
-                    for (int c2 = 0; c2 < nslots; ++c2)
-                        if (c2 != a && c2 != b)
-                            order[2 + rest++] = slots[c2];
-                    found = true;
-                }
+        int best = -1;
+        for (int a = 0; a < nslots; ++a)
+            for (int b = a + 1; b < nslots; ++b)
+            {
+                const int pa = FS.sbits[slots[a]], pb = FS.sbits[slots[b]];
+                const int score = direct ? (pa < kLowBits) + (pb < kLowBits) : 0;
+                if (pa % mod == pb % mod || score <= best)
+                    continue;
+                best = score;
+                int rest = 0;
+                order[0] = slots[a];
+                order[1] = slots[b];
+                for (int c2 = 0; c2 < nslots; ++c2)
+                    if (c2 != a && c2 != b)
+                        order[2 + rest++] = slots[c2];
+            }
         uint8_t perm = 0;
         uint32_t tensor_mask = 0;
         for (int b = 0; b < width; ++b)
@@ -770,40 +828,41 @@ double tensor_pass_cost(const TPassParams &tp, int amp_bytes)
     return tp.width == 3 ? 2.8 + 1.55 * tp.nstages : 2.0 + 3.1 * tp.nstages;
 }
 
+namespace
+{
+
+// Warps per chunk of an 8 x 8 pass (see tensor3_pass_kernel).
+int warps_for(uint64_t chunks) { return chunks <= 256 ? 8 : 4; }
+
+// One tensor kernel over the pass's chunks, as many CTAs as fit at once.
+template <typename K>
+int launch_chunks(K kernel, int threads, size_t smem, const TPassParams &tp, cudaStream_t stream)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    QCSB_CUDA(cudaGetDevice(&dev));
+    QCSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    QCSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    const uint64_t grid = std::min<uint64_t>(tp.chunks, static_cast<uint64_t>(sms) * std::max(per_sm, 1));
+    kernel<<<static_cast<unsigned>(grid), threads, smem, stream>>>(tp);
+    QCSB_CUDA(cudaGetLastError());
+    return 1;
+}
+
+} // namespace
+
 template <typename R>
 int launch_tensor_pass(const TPassParams &tp, cudaStream_t stream)
 {
     typedef typename Tensor<R>::V V;
     if (tp.reg_mats > 0 && tp.width != 3)
         throw std::runtime_error("internal: batched tensor passes run 8 x 8 stages only");
-    const size_t smem = kTensor4Buffers * sizeof(V) * kChunk;
-    const size_t smem3 = kTensor3Buffers * sizeof(V) * kChunk;
-    static bool configured[64] = {};
-    int dev = 0, sms = 0, per_sm = 0;
-    QCSB_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev])
-    {
-        QCSB_CUDA(cudaFuncSetAttribute(tensor_pass_kernel<R, kTensor4Buffers>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        QCSB_CUDA(cudaFuncSetAttribute(tensor3_pass_kernel<R, kTensor3Buffers>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem3)));
-        if (dev >= 0 && dev < 64)
-            configured[dev] = true;
-    }
-    QCSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (tp.width == 3)
-        QCSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tensor3_pass_kernel<R, kTensor3Buffers>,
-                                                                kThreads, smem3));
-    else
-        QCSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tensor_pass_kernel<R, kTensor4Buffers>,
-                                                                kThreads, smem));
-    const uint64_t grid = std::min<uint64_t>(tp.chunks, static_cast<uint64_t>(sms) * std::max(per_sm, 1));
-    if (tp.width == 3)
-        tensor3_pass_kernel<R, kTensor3Buffers><<<static_cast<unsigned>(grid), kThreads, smem3, stream>>>(tp);
-    else
-        tensor_pass_kernel<R, kTensor4Buffers><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(tp);
-    QCSB_CUDA(cudaGetLastError());
-    return 1;
+    const size_t smem = sizeof(V) * kChunk;
+    // (32 KiB at most: no opt-in needed)
+    if (tp.width != 3)
+        return launch_chunks(tensor_pass_kernel<R>, kThreads, smem, tp, stream);
+    const int w = warps_for(tp.chunks);
+    return w == 8 ? launch_chunks(tensor3_pass_kernel<R, 8>, 256, smem, tp, stream)
+                  : launch_chunks(tensor3_pass_kernel<R, 4>, 128, smem, tp, stream);
 }
 template int launch_tensor_pass<double>(const TPassParams &, cudaStream_t);
 template int launch_tensor_pass<float>(const TPassParams &, cudaStream_t);
