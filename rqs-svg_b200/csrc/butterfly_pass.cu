@@ -14,8 +14,11 @@
 //
 // Memory: thread t holds 16 amplitudes that differ in the stage's bits. When
 // the first (last) stage leaves local bits 0..2 alone, eight threads hold
-// whole 128- (64-) byte runs and load (store) the register directly: a
-// two-stage pass crosses shared memory once. The 28-qubit QFT with 1024 shots
+// whole 128- (64-) byte runs: each loads straight to its own slots (stores
+// straight from registers), and a two-stage pass has two barriers per chunk.
+// For complex128 the next chunk streams into the buffer during this one's
+// last stage (28-qubit flush 9.85 -> 9.35 ms); complex64 loads to registers
+// (with it 7.11 -> 7.38 ms). The 28-qubit QFT with 1024 shots
 // went from 16.9 to 11.3 ms (four passes of about 2.5 ms), its error against
 // 64 bits from 4.1e-15 to 2.2e-15.
 // One chunk buffer per CTA, four (complex64: eight) CTAs per SM.
@@ -37,33 +40,37 @@ constexpr int kThreads = 1 << (kTensorLocal - kStageBits);
 constexpr double kRsqrt2 = 0.70710678118654752440;   // the entries of gate_matrix's H
 
 // One run's table-fed factors: E[0] on every slot, E[1 + b] on the slots with
-// stage bit b (layout as for F_PRUN).
+// stage bit b (layout as for F_PRUN). The chunk's part of factor e is the
+// same for the whole CTA: lane e of each warp multiplies it together (its
+// loads in flight with the other lanes') and hands it round, instead of every
+// thread reading up to four tables per factor.
+template <typename V>
+__device__ __forceinline__ V from_lane(V v, int lane)
+{
+    return V{__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane)};
+}
+
 template <typename V>
 __device__ __forceinline__ void apply_run(V (&a)[R], const BRun &run, const double2 *tables, uint64_t chunk, int tid)
 {
-    const uint64_t packed = run.packed;
+    const uint32_t lm = static_cast<uint32_t>(run.packed) & 31u;
+    V part = V{1, 0};
+    const int lane = tid & 31;
+    if (lane <= kStageBits)
+        for (int g = 0; g < run.groups; ++g)
+            if ((run.packed >> (kChunkGroupBits * (g + 1) + lane)) & 1)
+            {
+                const uint32_t idx = static_cast<uint32_t>(chunk >> (kChunkGroupBits * g)) & ((1u << kChunkGroupBits) - 1);
+                part = cmul(cvt<V>(__ldg(tables + run.group_table[g][lane] + idx)), part);
+            }
 #pragma unroll
     for (int e = 0; e <= kStageBits; ++e)
     {
         if (!((run.used >> e) & 1))
             continue;
-        const uint32_t below = (1u << e) - 1u;
-        uint32_t off = run.table;
-        V f = V{1, 0};
-        const uint32_t lm = static_cast<uint32_t>(packed) & 31u;
+        V f = from_lane(part, e);
         if ((lm >> e) & 1)
-            f = cvt<V>(__ldg(tables + off + __popc(lm & below) * kThreads + tid));
-        off += __popc(lm) * kThreads;
-        for (int g = 0; g < kMaxChunkGroups; ++g)
-        {
-            const uint32_t gm = static_cast<uint32_t>(packed >> (kChunkGroupBits * (g + 1))) & 31u;
-            if ((gm >> e) & 1)
-            {
-                const uint32_t idx = static_cast<uint32_t>(chunk >> (kChunkGroupBits * g)) & ((1u << kChunkGroupBits) - 1);
-                f = cmul(cvt<V>(__ldg(tables + off + (__popc(gm & below) << kChunkGroupBits) + idx)), f);
-            }
-            off += __popc(gm) << kChunkGroupBits;
-        }
+            f = cmul(cvt<V>(__ldg(tables + run.thread_table[e] + tid)), f);
 #pragma unroll
         for (int r = 0; r < R; ++r)
             if (e == 0 || ((r >> (e > 0 ? e - 1 : 0)) & 1))
@@ -115,50 +122,93 @@ __global__ void __launch_bounds__(kThreads, sizeof(Real) == 8 ? 4 : 8)
                 off |= p.qbit[direct ? S.sbits[b] : kTensorLocal - kStageBits + b];
         return off;
     };
-
-    for (uint64_t c = blockIdx.x; c < p.chunks; c += gridDim.x)
+    // shared-memory position of a stage's slot r
+    struct Slots
     {
-        uint64_t cbase = c;
+        uint32_t p0, bit[kStageBits];
+        __device__ __forceinline__ uint32_t operator()(int r) const
+        {
+            uint32_t q = p0;
+#pragma unroll
+            for (int b = 0; b < kStageBits; ++b)
+                if ((r >> b) & 1)
+                    q ^= bit[b];
+            return q;
+        }
+    };
+    auto slots_of = [&](const BStage &S) {
+        Slots w;
+        w.p0 = static_cast<uint32_t>(swz<V>(static_cast<int>(slot0(S))));
+#pragma unroll
+        for (int b = 0; b < kStageBits; ++b)
+            w.bit[b] = static_cast<uint32_t>(swz<V>(1 << S.sbits[b]));
+        return w;
+    };
+    auto chunk_base = [&](uint64_t c) {
         for (int i = 0; i < kTensorLocal; ++i)
         {
-            const uint64_t lo = cbase & p.qmasks[i];
-            cbase = lo | ((cbase ^ lo) << 1);
+            const uint64_t lo = c & p.qmasks[i];
+            c = lo | ((c ^ lo) << 1);
         }
+        return c;
+    };
+    // the chunk's amplitudes on their way to shared memory: directly to the
+    // first stage's slots of the same thread, or in order
+    auto issue_load = [&](uint64_t base) {
+        const V *src = state + (base | in_off);
+        const Slots w = slots_of(p.stages[0]);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            cp_async_amp<V>(sb + (p.direct_in ? w(r) : swz<V>(tid + r * kThreads)),
+                            src + slot_offset(r, p.direct_in, p.stages[0]));
+        cp_async_commit();
+    };
+
+    const Real scale = static_cast<Real>(p.scale);
+    uint64_t c = blockIdx.x;
+    if (c >= p.chunks)
+        return;
+    uint64_t cbase = chunk_base(c);
+    // straight to registers where nothing is left to stream behind, and for
+    // complex64 (whose eight CTAs per SM overlap loads and stages as they are)
+    const bool to_registers = p.direct_in && (sizeof(Real) == 4 || p.chunks <= gridDim.x);
+    if (!to_registers)
+        issue_load(cbase);
+    for (; c < p.chunks; c += gridDim.x)
+    {
+        const uint64_t next = c + gridDim.x;
+        const uint64_t cbase_next = next < p.chunks ? chunk_base(next) : cbase;
         V a[R];
+        if (to_registers)
         {
             const V *src = state + (cbase | in_off);
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                a[r] = __ldcg(src + slot_offset(r, p.direct_in, p.stages[0]));
+                a[r] = __ldcg(src + slot_offset(r, true, p.stages[0]));
         }
-        if (!p.direct_in)
+        else
         {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                sb[swz<V>(tid + r * kThreads)] = a[r];
-            __syncthreads();
+            cp_async_wait<0>();
+            if (!p.direct_in)
+                __syncthreads();
         }
         for (int st = 0; st <= last; ++st)
         {
             const BStage &S = p.stages[st];
-            const uint32_t p0 = static_cast<uint32_t>(swz<V>(static_cast<int>(slot0(S))));
-            uint32_t sbit[kStageBits];
-#pragma unroll
-            for (int b = 0; b < kStageBits; ++b)
-                sbit[b] = static_cast<uint32_t>(swz<V>(1 << S.sbits[b]));
-            auto pos_of = [&](int r) {
-                uint32_t q = p0;
-#pragma unroll
-                for (int b = 0; b < kStageBits; ++b)
-                    if ((r >> b) & 1)
-                        q ^= sbit[b];
-                return q;
-            };
-            if (st > 0 || !p.direct_in)
+            const Slots w = slots_of(S);
+            if (st > 0 || !to_registers)
             {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    a[r] = sb[pos_of(r)];
+                    a[r] = sb[w(r)];
+            }
+            if (st == last && p.direct_out && next < p.chunks)
+            {
+                // the buffer is free: the next chunk streams in during this
+                // chunk's last stage
+                __syncthreads();
+                if (!to_registers)
+                    issue_load(cbase_next);
             }
             // steps: the diagonals before the first H, then bits 3 .. 0
 #pragma unroll
@@ -200,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(Real) == 8 ? 4 : 8)
             {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    sb[pos_of(r)] = a[r];
+                    sb[w(r)] = a[r];
                 __syncthreads();
             }
         }
@@ -209,15 +259,18 @@ __global__ void __launch_bounds__(kThreads, sizeof(Real) == 8 ? 4 : 8)
 #pragma unroll
             for (int r = 0; r < R; ++r)
                 a[r] = sb[swz<V>(tid + r * kThreads)];
+            if (next < p.chunks)
+            {
+                __syncthreads();
+                if (!to_registers)
+                    issue_load(cbase_next);
+            }
         }
-        const Real scale = static_cast<Real>(p.scale);
         V *dst = state + (cbase | out_off);
 #pragma unroll
         for (int r = 0; r < R; ++r)
             __stcs(dst + slot_offset(r, p.direct_out, p.stages[last]), V{a[r].x * scale, a[r].y * scale});
-        // every thread has read the buffer before the next chunk's writes
-        if (last > 0 || !p.direct_in || !p.direct_out)
-            __syncthreads();
+        cbase = cbase_next;
     }
 }
 
@@ -291,9 +344,26 @@ bool make_butterfly_params(const FPassParams &prm, int amp_bytes, BPassParams &b
                 {
                     if (step.run.used)
                         return false;
-                    step.run.packed = op.gcmask;
-                    step.run.table = op.lcval;
-                    step.run.used = op.b0;
+                    // the tables as an F_PRUN stores them: the thread tables,
+                    // then each chunk group's, factors ascending
+                    BRun &run = step.run;
+                    run.packed = op.gcmask;
+                    run.used = op.b0;
+                    uint32_t off = op.lcval;
+                    for (int e = 0; e <= kStageBits; ++e)
+                        if ((run.packed >> e) & 1)
+                        {
+                            run.thread_table[e] = off;
+                            off += kThreads;
+                        }
+                    for (int g = 0; g < kMaxChunkGroups; ++g)
+                        for (int e = 0; e <= kStageBits; ++e)
+                            if ((run.packed >> (kChunkGroupBits * (g + 1) + e)) & 1)
+                            {
+                                run.group_table[g][e] = off;
+                                off += 1u << kChunkGroupBits;
+                                run.groups = g + 1;
+                            }
                 }
                 continue;
             }

@@ -161,9 +161,11 @@ constexpr int kButterflyStages = 8;
 constexpr int kButterflyEntries = 256;
 struct BRun
 {
-    uint64_t packed;   // tables as an F_PRUN's: gcmask, lcval, b0
-    uint32_t table;
-    uint32_t used;
+    uint64_t packed;   // which factors have which tables, as an F_PRUN's gcmask
+    uint32_t used;     // which factors can differ from 1
+    int groups;        // chunk groups with a table: below this
+    uint32_t thread_table[kStageBits + 1];                 // offsets of the tables there are
+    uint32_t group_table[kMaxChunkGroups][kStageBits + 1];
 };
 struct BStep
 {
