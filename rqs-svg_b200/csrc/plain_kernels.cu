@@ -253,6 +253,82 @@ int launch_plain_dispatch(typename Cx<R>::T *state, int n, const GateOp &op, cud
     }
 }
 
+// ---------------------------------------------------------- small registers
+
+// A run of gates on a register of at most kSmallQubits qubits: one block holds
+// it in shared memory and applies the gates one after another, each with the
+// plain kernel's formula (bit-identical to it). A kernel per gate cost a
+// launch (3.7 us of host time) for a few hundred bytes of work.
+constexpr int kSmallQubits = 8;
+constexpr int kSmallThreads = 128;
+constexpr int kSmallOps = 32;        // per launch: parameters of 3 KiB (larger blocks launch slower)
+constexpr int kSmallEntries = 128;
+
+struct SmallOp
+{
+    uint8_t nops, na, diag, pad;
+    uint16_t entry, cval;
+    uint16_t off[4];
+    uint8_t masks[kSmallQubits];   // insertion masks below each operand position, ascending
+};
+
+template <typename R>
+struct SmallParams
+{
+    typedef typename Cx<R>::T V;
+    V *state;
+    int n, count;
+    SmallOp ops[kSmallOps];
+    V entries[kSmallEntries];
+};
+
+template <typename R>
+__global__ void __launch_bounds__(kSmallThreads) small_register_kernel(const __grid_constant__ SmallParams<R> p)
+{
+    typedef typename Cx<R>::T V;
+    __shared__ V amp[1 << kSmallQubits];
+    for (int i = threadIdx.x; i < (1 << p.n); i += kSmallThreads)
+        amp[i] = p.state[i];
+    __syncthreads();
+    for (int k = 0; k < p.count; ++k)
+    {
+        const SmallOp &op = p.ops[k];
+        const int na = op.na;
+        for (int g = threadIdx.x; g < (1 << (p.n - op.nops)); g += kSmallThreads)
+        {
+            uint32_t base = static_cast<uint32_t>(g);
+            for (int i = 0; i < op.nops; ++i)
+            {
+                const uint32_t lo = base & op.masks[i];
+                base = lo | ((base ^ lo) << 1);
+            }
+            base |= op.cval;
+            V v[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                if (a < na)
+                    v[a] = amp[base | op.off[a]];
+            for (int a = 0; a < na; ++a)
+            {
+                V acc = make_cx<V>(0.0, 0.0);
+                if (op.diag)
+                    acc = cmul(p.entries[op.entry + a], amp[base | op.off[a]]);
+                else
+                {
+#pragma unroll
+                    for (int b = 0; b < 4; ++b)
+                        if (b < na)
+                            acc = cfma(p.entries[op.entry + a * na + b], v[b], acc);
+                }
+                amp[base | op.off[a]] = acc;
+            }
+        }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < (1 << p.n); i += kSmallThreads)
+        p.state[i] = amp[i];
+}
+
 // ------------------------------------------------------------ preparation
 
 template <typename V>
@@ -814,6 +890,57 @@ int launch_gate_plain(typename Cx<R>::T *state, int n, const GateOp &op, cudaStr
 }
 
 template <typename R>
+int launch_gates_small(typename Cx<R>::T *state, int n, const GateOp *ops, size_t count, cudaStream_t stream)
+{
+    typedef typename Cx<R>::T V;
+    if (n > kSmallQubits)
+        throw std::runtime_error("internal: register too large for the small-register kernel");
+    int launches = 0;
+    SmallParams<R> p;
+    std::memset(&p, 0, sizeof(p));
+    p.state = state;
+    p.n = n;
+    int entries = 0;
+    auto flush = [&]() {
+        if (p.count == 0)
+            return;
+        small_register_kernel<R><<<1, kSmallThreads, 0, stream>>>(p);
+        QCSB_CUDA(cudaGetLastError());
+        ++launches;
+        p.count = entries = 0;
+    };
+    for (size_t k = 0; k < count; ++k)
+    {
+        const GateOp &op = ops[k];
+        if (op.na == 0)
+            continue;
+        const int ne = op.diag ? op.na : op.na * op.na;
+        if (p.count == kSmallOps || entries + ne > kSmallEntries)
+            flush();
+        SmallOp &o = p.ops[p.count++];
+        uint64_t masks[kMaxOps];
+        o.nops = static_cast<uint8_t>(fill_masks(op, masks));
+        for (int i = 0; i < o.nops; ++i)
+            o.masks[i] = static_cast<uint8_t>(masks[i]);
+        o.na = static_cast<uint8_t>(op.na);
+        o.diag = op.diag;
+        o.entry = static_cast<uint16_t>(entries);
+        o.cval = static_cast<uint16_t>(op.cval);
+        for (int a = 0; a < op.na; ++a)
+        {
+            o.off[a] = 0;
+            for (int i = 0; i < op.nt; ++i)
+                if ((op.act[a] >> i) & 1)
+                    o.off[a] |= static_cast<uint16_t>(1u << op.tq[i]);
+        }
+        for (int e = 0; e < ne; ++e)
+            p.entries[entries++] = make_cx<V>(op.mat[e].re, op.mat[e].im);
+    }
+    flush();
+    return launches;
+}
+
+template <typename R>
 int launch_init_zero(typename Cx<R>::T *state, int n, cudaStream_t stream)
 {
     typedef typename Cx<R>::T V;
@@ -974,6 +1101,7 @@ int launch_narrow(const double2 *in, uint64_t count, typename Cx<R>::T *out, cud
 
 #define QCSB_INSTANTIATE(R)                                                                                         \
     template int launch_gate_plain<R>(Cx<R>::T *, int, const GateOp &, cudaStream_t);                               \
+    template int launch_gates_small<R>(Cx<R>::T *, int, const GateOp *, size_t, cudaStream_t);                      \
     template int launch_init_zero<R>(Cx<R>::T *, int, cudaStream_t);                                                \
     template int launch_init_flat<R>(Cx<R>::T *, int, cudaStream_t);                                                \
     template int launch_init_sequential<R>(Cx<R>::T *, int, cudaStream_t);                                          \

@@ -103,6 +103,10 @@ GateOp make_gate_op(const GateMatrix &g, const int *tq, uint64_t cmask, uint64_t
 template <typename R>
 int launch_gate_plain(typename Cx<R>::T *state, int n, const GateOp &op, cudaStream_t stream);
 
+// A run of gates on a register of at most 8 qubits, 32 gates per kernel.
+template <typename R>
+int launch_gates_small(typename Cx<R>::T *state, int n, const GateOp *ops, size_t count, cudaStream_t stream);
+
 // |0..0>, flat (all 1), sequential (a[i] = i), and "entangled" (a[0] = 1,
 // leaving the rest as is) state preparation.
 template <typename R>
