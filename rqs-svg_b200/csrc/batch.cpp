@@ -117,6 +117,7 @@ void Batch::release_device()
     cudaFree(fill_regs_dev_);
     cudaFree(recipes_dev_);
     cudaFree(consts_dev_);
+    mats_cap_ = fill_regs_cap_ = recipes_cap_ = consts_cap_ = 0;
     params_dev_ = nullptr;
     fill_regs_dev_ = nullptr;
     recipes_dev_ = nullptr;
@@ -343,6 +344,23 @@ void Batch::make_recipe(Group &g)
         }
 }
 
+// Grow a device buffer to hold count elements (with room to spare: the
+// tuner's candidates differ a little in size, and an allocation for each of
+// them was most of a first run).
+template <typename T>
+void Batch::reserve(T *&buf, uint64_t &cap, uint64_t count)
+{
+    if (count <= cap && buf != nullptr)
+        return;
+    QCSB_CUDA(cudaStreamSynchronize(stream_));
+    cudaFree(buf);
+    buf = nullptr;
+    cap = 0;
+    const uint64_t want = count + count / 2;
+    QCSB_CUDA(cudaMalloc(&buf, sizeof(T) * want));
+    cap = want;
+}
+
 void Batch::layout_entries()
 {
     uint64_t off = 0;
@@ -351,15 +369,7 @@ void Batch::layout_entries()
         g.mats_off = off;
         off += (uint64_t)g.stride * g.members.size();
     }
-    if (off != mats_count_ || mats_dev_ == nullptr)
-    {
-        if (stream_)
-            QCSB_CUDA(cudaStreamSynchronize(stream_));
-        cudaFree(mats_dev_);
-        mats_dev_ = nullptr;
-        mats_count_ = off;
-        QCSB_CUDA(cudaMalloc(&mats_dev_, sizeof(double2) * std::max<uint64_t>(off, 1)));
-    }
+    reserve(mats_dev_, mats_cap_, std::max<uint64_t>(off, 1));
     for (Group &g : groups_)
         for (Pass &p : g.passes)
         {
@@ -383,17 +393,11 @@ void Batch::upload_recipes()
         recipes.insert(recipes.end(), g.recipe.begin(), g.recipe.end());
         consts.insert(consts.end(), g.consts.begin(), g.consts.end());
     }
-    if (stream_)
-        QCSB_CUDA(cudaStreamSynchronize(stream_));
-    cudaFree(fill_regs_dev_);
-    cudaFree(recipes_dev_);
-    cudaFree(consts_dev_);
-    fill_regs_dev_ = nullptr;
-    recipes_dev_ = nullptr;
-    consts_dev_ = nullptr;
-    QCSB_CUDA(cudaMalloc(&fill_regs_dev_, sizeof(BatchFillReg) * regs.size()));
-    QCSB_CUDA(cudaMalloc(&recipes_dev_, sizeof(BatchEntry) * std::max<size_t>(recipes.size(), 1)));
-    QCSB_CUDA(cudaMalloc(&consts_dev_, sizeof(double2) * consts.size()));
+    reserve(fill_regs_dev_, fill_regs_cap_, regs.size());
+    reserve(recipes_dev_, recipes_cap_, std::max<size_t>(recipes.size(), 1));
+    reserve(consts_dev_, consts_cap_, consts.size());
+    // (the buffers may still be read by the last candidate's fill)
+    QCSB_CUDA(cudaStreamSynchronize(stream_));
     QCSB_CUDA(cudaMemcpy(fill_regs_dev_, regs.data(), sizeof(BatchFillReg) * regs.size(), cudaMemcpyHostToDevice));
     QCSB_CUDA(cudaMemcpy(recipes_dev_, recipes.data(), sizeof(BatchEntry) * recipes.size(), cudaMemcpyHostToDevice));
     QCSB_CUDA(cudaMemcpy(consts_dev_, consts.data(), sizeof(double2) * consts.size(), cudaMemcpyHostToDevice));
@@ -568,7 +572,6 @@ void Batch::build()
     if (stream_)
         QCSB_CUDA(cudaStreamSynchronize(stream_));
     release_device();
-    mats_count_ = 0;
     groups_.clear();
     // group by structure
     for (uint32_t ci = 0; ci < circuits_.size(); ++ci)

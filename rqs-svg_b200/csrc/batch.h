@@ -141,6 +141,8 @@ class Batch
     void ensure_tensor_mats();
     void layout_entries();
     void make_recipe(Group &g);
+    template <typename T>
+    void reserve(T *&buf, uint64_t &cap, uint64_t count);
     void upload_recipes();
     void upload_params();
     int fill_entries(int only_group = -1);
@@ -167,7 +169,7 @@ class Batch
     BatchFillReg *fill_regs_dev_ = nullptr;
     BatchEntry *recipes_dev_ = nullptr;
     double2 *consts_dev_ = nullptr;
-    uint64_t mats_count_ = 0;
+    uint64_t mats_cap_ = 0, fill_regs_cap_ = 0, recipes_cap_ = 0, consts_cap_ = 0;   // elements
     BatchZItem *zitems_dev_ = nullptr;
     BatchZReg *zregs_dev_ = nullptr;
     uint32_t num_zitems_ = 0;

@@ -2304,6 +2304,15 @@ FusedExecutor::FlushPlan *FusedExecutor::find_plan(const std::vector<GateOp> &qu
     return nullptr;
 }
 
+// Bytes of one matrix of a tensor pass in its format: 8 x 8 mma.sync
+// fragments, 16 x 16 mma.sync fragments, or tcgen05 slabs (high and low).
+static size_t tensor_matrix_bytes(const TPassParams &tp)
+{
+    if (tp.umma)
+        return 2 * static_cast<size_t>(kUmmaSlab);
+    return static_cast<size_t>(tp.width == 3 ? kTensor3Fragments : kTensorFragments) * 32 * 16;
+}
+
 // One launch of a plan: a plain gate kernel, a register pass, or a tensor
 // pass (its stage-matrix builder, then the pass).
 int FusedExecutor::launch_plan_step(FlushPlan &plan, long st, void *state, const double2 *tables_dev,
@@ -2343,15 +2352,18 @@ int FusedExecutor::launch_plan_step(FlushPlan &plan, long st, void *state, const
         }
         else
         {
-            if (tb.nmats > mats_cap_)
+            const size_t need = tb.nmats * tensor_matrix_bytes(tp);
+            if (need > mats_cap_)
             {
                 // the old buffer may still be read by queued passes
                 QCSB_CUDA(cudaStreamSynchronize(stream_));
                 cudaFree(mats_dev_);
                 mats_dev_ = nullptr;
                 mats_cap_ = 0;
-                const size_t cap = std::max<size_t>(tb.nmats, 256);
-                QCSB_CUDA(cudaMalloc(&mats_dev_, cap * kTensorMatrixBytes));
+                // (a small first buffer: 2 MiB at once took the first flush
+                // of a small register 0.2 ms longer)
+                const size_t cap = std::max<size_t>(2 * need, size_t(256) << 10);
+                QCSB_CUDA(cudaMalloc(&mats_dev_, cap));
                 mats_cap_ = cap;
             }
             mats = mats_dev_;
@@ -2389,15 +2401,6 @@ int FusedExecutor::launch_plan_step(FlushPlan &plan, long st, void *state, const
     return launches;
 }
 
-// Bytes of one matrix of a tensor pass in its format: 8 x 8 mma.sync
-// fragments, 16 x 16 mma.sync fragments, or tcgen05 slabs (high and low).
-static size_t tensor_matrix_bytes(const TPassParams &tp)
-{
-    if (tp.umma)
-        return 2 * static_cast<size_t>(kUmmaSlab);
-    return static_cast<size_t>(tp.width == 3 ? kTensor3Fragments : kTensorFragments) * 32 * 16;
-}
-
 int FusedExecutor::replay(FlushPlan &plan, void *state, qcs_b200_stats &stats, KernelTimer &timer)
 {
     if (plan.mats == nullptr && !plan.tparams.empty())
@@ -2413,10 +2416,12 @@ int FusedExecutor::replay(FlushPlan &plan, void *state, qcs_b200_stats &stats, K
         }
         // kept matrices are a cache: they are made only while 256 MiB stay
         // free beside them, so that they never take the memory the
-        // register's own scratch (sampler, staging) would need later
+        // register's own scratch (sampler, staging) would need later; up to
+        // 512 KiB without asking (the question takes longer than the builds)
         size_t free_b = 0, total_b = 0;
-        const bool room = total <= kKeptMatsBytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-                          free_b >= total + kKeptMatsFreeReserve;
+        const bool room = total <= kKeptMatsSmall ||
+                          (total <= kKeptMatsBytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+                           free_b >= total + kKeptMatsFreeReserve);
         if (!room || cudaMalloc(&plan.mats, total) != cudaSuccess)
         {
             plan.mats = nullptr;

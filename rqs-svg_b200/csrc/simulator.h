@@ -291,6 +291,7 @@ class FusedExecutor
         }
     };
     static constexpr size_t kKeptMatsBytes = size_t(256) << 20;   // device memory of one kept plan's matrices
+    static constexpr size_t kKeptMatsSmall = size_t(512) << 10;   // kept whatever is free
     static constexpr size_t kKeptMatsFreeReserve = size_t(256) << 20;   // left free beside kept matrices
     void settle_judge();
     const double2 *upload_tables(const std::vector<double2> &tables);
@@ -320,7 +321,7 @@ class FusedExecutor
     // matrices of the tensor pass being run: every pass's builder writes
     // them right before the pass reads them, in stream order
     double2 *mats_dev_ = nullptr;
-    size_t mats_cap_ = 0;   // matrices
+    size_t mats_cap_ = 0;   // bytes
     CostModel *model_ = nullptr;
     // "measured device time is the judge": per queue signature, the device
     // time of a flush under each planner; once both are known the faster one
