@@ -2428,7 +2428,13 @@ int FusedExecutor::replay(FlushPlan &plan, void *state, qcs_b200_stats &stats, K
             (void)cudaGetLastError();   // no room: keep building into the shared buffer
         }
     }
-    const double2 *tables_dev = upload_tables(plan.tables);
+    // the phase-run tables, for passes that run from them and for matrices
+    // that are still to be built (kept ones hold their factors; without the
+    // copy and its event an 11-qubit ansatz loop took 1571 -> 1389 us)
+    bool use_tables = !plan.mats_built;
+    for (int t : plan.tensor_of)
+        use_tables = use_tables || t < 0;
+    const double2 *tables_dev = use_tables ? upload_tables(plan.tables) : nullptr;
     int launches = 0;
     for (long st : plan.steps)
         launches += launch_plan_step(plan, st, state, tables_dev, stats, timer, nullptr);

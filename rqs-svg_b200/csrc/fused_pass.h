@@ -101,10 +101,6 @@ struct TBuildParams
     uint32_t reg0;               // first register of this launch (grid.y covers at most 65535)
     TStage stages[kFusedMaxStages];
 };
-// bytes of the matrix buffer per matrix, either format
-constexpr size_t kTensorMatrixBytes =
-    kTensorFragments * 32 * 16 > 2 * kUmmaSlab ? kTensorFragments * 32 * 16 : 2 * kUmmaSlab;
-
 struct TPassParams
 {
     void *state;

@@ -464,7 +464,8 @@ __device__ __forceinline__ double2 block_sum_partials(const double2 *partials, i
 // writes (P0, P1) to p.result. A chain of measurements halves the groups at
 // every step, and most of its reductions are bound by latency: a block per
 // 2048 groups (eight per thread, four of them in flight), and with one block
-// no partials and no ticket.
+// no partials and no ticket (9.0 -> 6.8 us for the last ones of a 20-qubit
+// chain under the profiler).
 constexpr int kProbGroups = 4;   // groups in flight per thread
 
 template <typename R>
@@ -571,7 +572,9 @@ __global__ void collapse_mask_kernel(V *state, uint64_t count, uint64_t cmask, u
 // last of its 3.5 blocks per SM alone). Small registers are bound by
 // latency: up to one tile (11 or 12 qubits) one block writes the sums
 // itself; otherwise the second kernel adds the blocks' partials, a warp per
-// sum.
+// sum. Under the profiler: 800 -> 9 us at 11 qubits (one thread did it all),
+// 18 + 59 -> 5.5 + 9 at 17, 36 + 60 -> 17 + 9 at 22; complex128 at 27
+// qubits reads at 6.6 TB/s.
 constexpr int kZThreads = 256;
 constexpr int kZLoads = 8;
 constexpr int kZMaxBlocks = 296;                // two per SM

@@ -57,7 +57,8 @@ __device__ __forceinline__ double norm2(V a)
 
 // Leaf sums in physical order, so that the register is read in full lines
 // whatever the measurement order (a register in reversed order, as a QFT's
-// swaps leave it, read a 16-byte amplitude per 4 KiB before). Lane l of a warp
+// swaps leave it, read a 16-byte amplitude per 4 KiB before: 6.29 -> 0.71 ms at
+// 28 qubits, 6.1 TB/s). Lane l of a warp
 // holds physical bits 0..4; `rest` are the physical bits of the steps below
 // the leaves. A thread adds up the amplitudes that differ in the rest bits
 // above the lane's (the subsets h of rest_hi, kLeafLoads loads in flight),
@@ -141,8 +142,8 @@ __global__ void tree_level_kernel(double *tree, int d)
 // Levels top - 1 .. 10 from level `top` (11 .. 20). A node's children differ
 // in their highest bit, so the nodes below node p of level 10 are those with
 // p as their low ten bits: a block takes kColumns adjacent p and reduces
-// their columns in shared memory. One launch instead of one per level (each
-// 2.5-5 us).
+// their columns in shared memory. One launch of 10 us instead of one per level
+// (each 2.5-5 us).
 __global__ void __launch_bounds__(kThreads) tree_columns_kernel(double *tree, int top)
 {
     __shared__ double col[kMaxColumnRows][kColumns];
