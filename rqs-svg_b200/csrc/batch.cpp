@@ -172,6 +172,7 @@ uint32_t Batch::add_circuit(int n, const qcs_b200_gate *gates, uint32_t count)
         std::memcpy(g.name, in.name, sizeof(g.name));
         g.id = gate_id(g.name);
         g.np = gate_nparams(g.id);
+        g.formula = formula_of(g.name, g.np);
         const int arity = gate_arity(g.name);
         if (arity > 2)
             throw std::runtime_error(strformat("gate %u (%s): batches take gates on at most two targets", i, g.name));
@@ -331,7 +332,7 @@ void Batch::make_recipe(Group &g)
                 {
                     const uint64_t tag = static_cast<uint64_t>(m[e].x - kTag);
                     const Gate &gt = rep.gates[tag / 16];
-                    r = BatchEntry{formula_of(gt.name, gt.np), static_cast<uint8_t>(tag % 16), 0, param_of[tag / 16]};
+                    r = BatchEntry{gt.formula, static_cast<uint8_t>(tag % 16), 0, param_of[tag / 16]};
                     continue;
                 }
                 uint32_t ci = 0;
@@ -562,6 +563,27 @@ void Batch::tune()
     }
 }
 
+// Whether a circuit's gates can run by the plan and the recipe of a group:
+// the same ops entry for entry at the probe parameters, on the same
+// sub-indices, and every parametrised one by the same formula.
+bool Batch::same_structure(const Group &g, const Circuit &c, const std::vector<GateOp> &shape) const
+{
+    if (g.n != c.n || g.shape.size() != shape.size())
+        return false;
+    const Circuit &rep = circuits_[g.members.front()];
+    for (size_t i = 0; i < shape.size(); ++i)
+    {
+        const GateOp &a = g.shape[i], &b = shape[i];
+        if (rep.gates[i].formula != c.gates[i].formula || rep.gates[i].np != c.gates[i].np || a.nt != b.nt ||
+            a.na != b.na || a.diag != b.diag || a.cmask != b.cmask || a.cval != b.cval ||
+            std::memcmp(a.tq, b.tq, sizeof(a.tq[0]) * a.nt) != 0 ||
+            std::memcmp(a.act, b.act, sizeof(a.act[0]) * a.na) != 0 ||
+            std::memcmp(a.mat, b.mat, sizeof(a.mat[0]) * (a.diag ? a.na : a.na * a.na)) != 0)
+            return false;
+    }
+    return true;
+}
+
 void Batch::build()
 {
     if (circuits_.empty())
@@ -584,9 +606,12 @@ void Batch::build()
         {
             const GateMatrix gm = gate_matrix(gt.id, kProbe, gt.np);
             const GateOp op = make_gate_op(gm, gt.tq, gt.cmask, gt.cval);
-            sig = mix(sig, (uint64_t)op.nt | ((uint64_t)op.na << 8) | ((uint64_t)op.diag << 16) | ((uint64_t)gt.np << 24));
+            sig = mix(sig, (uint64_t)op.nt | ((uint64_t)op.na << 8) | ((uint64_t)op.diag << 16) | ((uint64_t)gt.np << 24) |
+                               ((uint64_t)gt.formula << 32));
             for (int i = 0; i < op.nt; ++i)
                 sig = mix(sig, (uint64_t)op.tq[i]);
+            for (int a = 0; a < op.na; ++a)
+                sig = mix(sig, (uint64_t)op.act[a]);
             sig = mix(mix(sig, op.cmask), op.cval);
             const int ne = op.diag ? op.na : op.na * op.na;
             for (int e = 0; e < ne; ++e)
@@ -596,7 +621,7 @@ void Batch::build()
         sig = mix(sig, c.gates.size());
         int gi = -1;
         for (int i = 0; i < (int)groups_.size(); ++i)
-            if (groups_[i].signature == sig && groups_[i].n == c.n && groups_[i].shape.size() == shape.size())
+            if (groups_[i].signature == sig && same_structure(groups_[i], c, shape))
                 gi = i;
         if (gi < 0)
         {

@@ -97,6 +97,7 @@ class Batch
         char name[16];
         int id;      // gate table index (looked up once, at add_circuit)
         int np;
+        BatchFormula formula;
         int tq[kMaxTargets];
         uint64_t cmask, cval;
     };
@@ -137,6 +138,7 @@ class Batch
 
     void invalidate();
     void build();
+    bool same_structure(const Group &g, const Circuit &c, const std::vector<GateOp> &shape) const;
     void plan_group(Group &g, int k, bool tensor = false);
     void ensure_tensor_mats();
     void layout_entries();

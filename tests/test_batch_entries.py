@@ -47,3 +47,31 @@ def test_batch_entries_match_oracle(gpu_lib, oracle_lib, name, precision):
         with qcs_b200.Simulator(oracle_lib, N) as sim:
             sim.run(ops)
             assert np.max(np.abs(got - sim.statevector())) <= tol
+
+
+@pytest.mark.parametrize("tensor", [0, 2])
+@pytest.mark.parametrize("precision", [128, 64])
+def test_gates_that_differ_in_their_sub_indices_only(gpu_lib, oracle_lib, precision, tensor):
+    """xx_plus_yy and xx_minus_yy have the same 2 x 2 block, on |01>, |10>
+    and on |00>, |11>: circuits that differ in nothing else have plans of
+    their own, while u3 and u, p and u1 share one. Tolerances as above."""
+    n = 11
+    pre = [("u3", (0.3 + q, 0.2, 0.9 - q), (q,), (), ()) for q in range(n)]
+    swapped = {"xx_plus_yy": "xx_minus_yy", "u3": "u", "p": "u1"}
+    a = pre + [("p", (0.4,), (3,), (), (1,)), ("xx_plus_yy", (0.7, 0.4), (2, 5), (), ()),
+               ("xx_plus_yy", (1.1, -0.6), (9, 0), (4,), (7,))]
+    b = [(swapped["xx_plus_yy"], *op[1:]) if op[0] == "xx_plus_yy" else op for op in a]
+    c = [(swapped[op[0]], *op[1:]) if op[0] in ("u3", "p") else op for op in a]
+    with qcs_b200.Batch(gpu_lib, precision) as batch:
+        batch.set_tensor_passes(tensor)
+        for circ in (a, b, c, b):
+            batch.add_circuit(n, circ)
+        batch.run()
+        assert batch.info()["groups"] == 2
+        states, z = [batch.statevector(i) for i in range(4)], batch.expectation_z()
+    tol = 1e-12 if precision == 128 else 5e-6
+    for i, circ in enumerate((a, b, c, b)):
+        with qcs_b200.Simulator(oracle_lib, n) as sim:
+            sim.run(circ)
+            assert np.max(np.abs(states[i] - sim.statevector())) <= tol, i
+            assert np.max(np.abs(z[i] - sim.expectation_z()[0])) <= tol, i
