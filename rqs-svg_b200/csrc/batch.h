@@ -131,7 +131,6 @@ class Batch
         uint32_t stride = 0;             // gate entries per register
         std::vector<BatchEntry> recipe;  // what they are
         std::vector<double2> consts;     // the recipe's constants
-        uint32_t first_reg = 0;          // of the group's registers in the fill list
         uint64_t mats_off = 0;           // first entry of the group's registers
         uint64_t amp_off = 0;            // first amplitude of the group's registers
     };
@@ -140,14 +139,14 @@ class Batch
     void build();
     bool same_structure(const Group &g, const Circuit &c, const std::vector<GateOp> &shape) const;
     void plan_group(Group &g, int k, bool tensor = false);
-    void ensure_tensor_mats();
-    void layout_entries();
+    void ensure_tensor_mats(size_t first, size_t last);
+    void layout_entries(size_t first, size_t last);
     void make_recipe(Group &g);
     template <typename T>
     void reserve(T *&buf, uint64_t &cap, uint64_t count);
-    void upload_recipes();
+    void upload_recipes(size_t first, size_t last);
     void upload_params();
-    int fill_entries(int only_group = -1);
+    int fill_entries();
     void enqueue_passes(const Group &g, cudaStream_t s, int *launches);
     void enqueue_group(int gi, cudaStream_t s, int *launches);
     void enqueue_results(cudaStream_t s, int *launches);
@@ -169,6 +168,7 @@ class Batch
     double2 *mats_dev_ = nullptr;
     double *params_dev_ = nullptr, *params_host_ = nullptr;
     BatchFillReg *fill_regs_dev_ = nullptr;
+    uint32_t num_fill_regs_ = 0;
     BatchEntry *recipes_dev_ = nullptr;
     double2 *consts_dev_ = nullptr;
     uint64_t mats_cap_ = 0, fill_regs_cap_ = 0, recipes_cap_ = 0, consts_cap_ = 0;   // elements

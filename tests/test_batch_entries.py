@@ -2,6 +2,8 @@
 at most two targets, with and without controls, before and after
 set_parameters, against the CPU oracle."""
 
+import time
+
 import numpy as np
 import pytest
 
@@ -75,3 +77,32 @@ def test_gates_that_differ_in_their_sub_indices_only(gpu_lib, oracle_lib, precis
             sim.run(circ)
             assert np.max(np.abs(states[i] - sim.statevector())) <= tol, i
             assert np.max(np.abs(z[i] - sim.expectation_z()[0])) <= tol, i
+
+
+def test_first_run_grows_with_the_number_of_structures(gpu_lib):
+    """A first run plans and tunes each structure by itself: four times as
+    many different circuits take about four times as long (measured 4.0; with
+    the entries of all structures uploaded for every candidate 9.4). The
+    smaller batch is the better of two, so that a slow first call does not
+    stand for it."""
+    rng = np.random.default_rng(2)
+    circuits = []
+    for _ in range(1200):
+        circ = []
+        for k in range(200):
+            a, b = (int(q) for q in rng.choice(N, 2, replace=False))
+            circ.append(("ry", (0.1 * k,), (a,), (), ()) if k % 2 else ("x", (), (a,), (), (b,)))
+        circuits.append(circ)
+
+    def first_run(count):
+        with qcs_b200.Batch(gpu_lib, 64) as batch:
+            for circ in circuits[:count]:
+                batch.add_circuit(N, circ)
+            t0 = time.perf_counter()
+            batch.run()
+            t = time.perf_counter() - t0
+            assert batch.info()["groups"] == count
+        return t
+
+    few = min(first_run(300), first_run(300))
+    assert first_run(1200) <= 6.5 * few
