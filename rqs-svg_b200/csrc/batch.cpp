@@ -345,25 +345,36 @@ void Batch::make_recipe(Group &g)
         }
 }
 
-// Grow a device buffer to hold count elements (with room to spare: the
-// tuner's candidates differ a little in size, and an allocation for each of
-// them was most of a first run).
+// Make a device buffer hold count elements. While tuning it grows with room
+// to spare where there is that much (candidates differ a little in size, and
+// an allocation for each of them was most of a first run); at the end a spare
+// of more than kSpareBytes is given back, so that a built batch holds what it
+// needs: a narrow register's entries take about as much memory as its
+// amplitudes.
 template <typename T>
-void Batch::reserve(T *&buf, uint64_t &cap, uint64_t count)
+void Batch::reserve(T *&buf, uint64_t &cap, uint64_t count, bool tuning)
 {
-    if (count <= cap && buf != nullptr)
+    constexpr uint64_t kSpareBytes = uint64_t(1) << 20;
+    if (buf != nullptr && count <= cap && (tuning || sizeof(T) * (cap - count) <= kSpareBytes))
         return;
     QCSB_CUDA(cudaStreamSynchronize(stream_));
     cudaFree(buf);
     buf = nullptr;
     cap = 0;
-    const uint64_t want = count + count / 2;
-    QCSB_CUDA(cudaMalloc(&buf, sizeof(T) * want));
+    uint64_t want = tuning ? count + count / 2 : count;
+    if (want > count && cudaMalloc(&buf, sizeof(T) * want) != cudaSuccess)
+    {
+        (void)cudaGetLastError();
+        buf = nullptr;
+        want = count;
+    }
+    if (buf == nullptr)
+        QCSB_CUDA(cudaMalloc(&buf, sizeof(T) * want));
     cap = want;
 }
 
 // The entry buffer laid out for groups [first, last).
-void Batch::layout_entries(size_t first, size_t last)
+void Batch::layout_entries(size_t first, size_t last, bool tuning)
 {
     uint64_t off = 0;
     for (size_t gi = first; gi < last; ++gi)
@@ -371,7 +382,7 @@ void Batch::layout_entries(size_t first, size_t last)
         groups_[gi].mats_off = off;
         off += (uint64_t)groups_[gi].stride * groups_[gi].members.size();
     }
-    reserve(mats_dev_, mats_cap_, std::max<uint64_t>(off, 1));
+    reserve(mats_dev_, mats_cap_, std::max<uint64_t>(off, 1), tuning);
     for (size_t gi = first; gi < last; ++gi)
         for (Pass &p : groups_[gi].passes)
         {
@@ -381,7 +392,7 @@ void Batch::layout_entries(size_t first, size_t last)
 }
 
 // The recipes, constants and fill list of groups [first, last), to the device.
-void Batch::upload_recipes(size_t first, size_t last)
+void Batch::upload_recipes(size_t first, size_t last, bool tuning)
 {
     std::vector<BatchFillReg> regs;
     std::vector<BatchEntry> recipes;
@@ -396,9 +407,9 @@ void Batch::upload_recipes(size_t first, size_t last)
         consts.insert(consts.end(), g.consts.begin(), g.consts.end());
     }
     num_fill_regs_ = static_cast<uint32_t>(regs.size());
-    reserve(fill_regs_dev_, fill_regs_cap_, regs.size());
-    reserve(recipes_dev_, recipes_cap_, std::max<size_t>(recipes.size(), 1));
-    reserve(consts_dev_, consts_cap_, consts.size());
+    reserve(fill_regs_dev_, fill_regs_cap_, regs.size(), tuning);
+    reserve(recipes_dev_, recipes_cap_, std::max<size_t>(recipes.size(), 1), tuning);
+    reserve(consts_dev_, consts_cap_, consts.size(), tuning);
     // (the buffers may still be read by the last candidate's fill)
     QCSB_CUDA(cudaStreamSynchronize(stream_));
     QCSB_CUDA(cudaMemcpy(fill_regs_dev_, regs.data(), sizeof(BatchFillReg) * regs.size(), cudaMemcpyHostToDevice));
@@ -543,9 +554,9 @@ void Batch::tune()
         for (const auto &cand : cands)
         {
             plan_group(g, cand.first, cand.second);
-            layout_entries(gi, gi + 1);
+            layout_entries(gi, gi + 1, true);
             ensure_tensor_mats(gi, gi + 1);
-            upload_recipes(gi, gi + 1);
+            upload_recipes(gi, gi + 1, true);
             fill_entries();
             int launches = 0;
             enqueue_passes(g, stream_, &launches);   // warm-up
@@ -691,9 +702,9 @@ void Batch::build()
 
     // plans: tuned per group, then the final entry layout
     tune();
-    layout_entries(0, groups_.size());
+    layout_entries(0, groups_.size(), false);
     ensure_tensor_mats(0, groups_.size());
-    upload_recipes(0, groups_.size());
+    upload_recipes(0, groups_.size(), false);
     fill_entries();
 
     // capture the run: a graph per group, then the results (after dropping

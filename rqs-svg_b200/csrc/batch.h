@@ -140,11 +140,11 @@ class Batch
     bool same_structure(const Group &g, const Circuit &c, const std::vector<GateOp> &shape) const;
     void plan_group(Group &g, int k, bool tensor = false);
     void ensure_tensor_mats(size_t first, size_t last);
-    void layout_entries(size_t first, size_t last);
+    void layout_entries(size_t first, size_t last, bool tuning);
     void make_recipe(Group &g);
     template <typename T>
-    void reserve(T *&buf, uint64_t &cap, uint64_t count);
-    void upload_recipes(size_t first, size_t last);
+    void reserve(T *&buf, uint64_t &cap, uint64_t count, bool tuning);
+    void upload_recipes(size_t first, size_t last, bool tuning);
     void upload_params();
     int fill_entries();
     void enqueue_passes(const Group &g, cudaStream_t s, int *launches);

@@ -106,3 +106,29 @@ def test_first_run_grows_with_the_number_of_structures(gpu_lib):
 
     few = min(first_run(300), first_run(300))
     assert first_run(1200) <= 6.5 * few
+
+
+def test_device_memory_of_a_batch_is_what_it_needs(gpu_lib):
+    """4000 registers of 10 qubits with 300 U3 gates each: the amplitudes
+    (64 MiB), at most four entries per gate (74 MiB), the parameters (28 MiB)
+    and 24 MiB for the work lists, the tuner's spare and the allocator's
+    granularity."""
+    import torch
+
+    count, gates = 4000, 300
+    rng = np.random.default_rng(1)
+    circ = [("u3", tuple(rng.uniform(-3, 3, 3)), (i % N,), (), ((i // N + i) % N,) if (i // N) % N else ()) for i in range(gates)]
+    circ = [op for op in circ if op[2] != op[4]]
+    with qcs_b200.Batch(gpu_lib, 128) as warm:   # what a first batch of the process loads
+        warm.add_circuit(N, circ)
+        warm.run()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with qcs_b200.Batch(gpu_lib, 128) as batch:
+        for _ in range(count):
+            batch.add_circuit(N, circ)
+        batch.run()
+        assert batch.info()["groups"] == 1
+        used = before - torch.cuda.mem_get_info()[0]
+    need = count * (16 * 2**N + 4 * 16 * len(circ) + 24 * len(circ))
+    assert used <= need + (24 << 20)
