@@ -1649,6 +1649,7 @@ bool build_tensor8(const std::vector<GateOp> &q, const PlannedPass &pp, int n, i
         ok = make_tensor_params(params[before + j], conds[before + j], amp_bytes, out.tparams[j], out.tbuild[j], 3);
         out.cost += ok ? tensor_pass_cost(out.tparams[j], amp_bytes) : 0.0;
         out.tensor.push_back(static_cast<int>(j));
+        out.butterfly.push_back(-1);
     }
     if (!ok)
     {
@@ -1661,9 +1662,8 @@ bool build_tensor8(const std::vector<GateOp> &q, const PlannedPass &pp, int n, i
     return ok;
 }
 
-// More multi-qubit phases than gates with dense targets (a QFT): the phases
-// reach too many qubits outside their stages to share a few matrices, and a
-// register pass runs them from tables.
+// More multi-qubit phases than gates with dense targets (a QFT, a Trotter
+// step).
 bool mostly_phases(const std::vector<GateOp> &q, const PlannedPass &pp)
 {
     size_t dense = 0, phases = 0;
@@ -1676,32 +1676,86 @@ bool mostly_phases(const std::vector<GateOp> &q, const PlannedPass &pp)
     return phases > dense;
 }
 
+// Hadamards and diagonals only: a pass that can run as a butterfly.
+bool hadamards_only(const std::vector<GateOp> &q, const PlannedPass &pp)
+{
+    for (int oi : pp.ops)
+        if (!q[oi].diag && !is_hadamard(q[oi]))
+            return false;
+    return true;
+}
+
+// What a complex128 pass with other gates costs at least other than as 8 x 8
+// stages, without building those forms: register_pass_cost asks no less than
+// this for each gate, and diagonals may cost next to nothing.
+double cost_floor(const std::vector<GateOp> &q, const PlannedPass &pp, int n)
+{
+    double gates = 0.0;
+    for (int oi : pp.ops)
+        if (const GateOp &op = q[oi]; !op.diag)
+            gates += op.nt == 1 ? (is_x(op) ? 0.5 : is_real(op) ? 0.325 : 0.65) : is_swap(op) ? 1.7 : 2.8;
+    int loc_of[kMaxQubits];
+    for (int b = 0, l = 0; b < kMaxQubits; ++b)
+        loc_of[b] = b < n && ((pp.local >> b) & 1) ? l++ : -1;
+    std::vector<std::vector<int>> ops;
+    std::vector<uint32_t> bits;
+    schedule_stages(q, pp, loc_of, ops, bits);
+    const double stages = static_cast<double>(ops.size());
+    return std::min(1.7 + 1.2 * stages + gates, 2.0 + 3.1 * stages);
+}
+
 } // namespace
 
 // How a planned pass runs: its pieces (built by build_pieces and already
 // appended to params / pieces / conds from index `before` on) on the
-// register path or as 16 x 16 tensor stages, per piece whichever the cost
+// register path (as butterflies where they are Hadamards and diagonals) or as
+// 16 x 16 tensor stages, per piece whichever the cost
 // estimate favours (tensor mode 1) or 16 x 16 wherever allowed (2); or the
 // same gates replanned with three dense bits per stage as 8 x 8 tensor
 // stages, which then replace those pieces: when the estimate favours them
-// (1) or wherever every piece allows them (3).
+// (1) or wherever every piece allows them (3). eight: the 8 x 8 form where
+// direct_tensor_pass left it, its pieces from index eight_at to `before`.
 void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
-                      size_t before, int engine)
+                      size_t before, int engine, PassChoice *eight, size_t eight_at)
 {
     out = PassChoice();
-    // automatic mode: below tensor_min_qubits a pass that small_tensor_pass
-    // did not take runs on the register path, as do complex128 passes of
-    // mostly phases
+    // drops pieces [first, last)
+    auto drop = [&](size_t first, size_t last) {
+        params.erase(params.begin() + first, params.begin() + last);
+        pieces.erase(pieces.begin() + first, pieces.begin() + last);
+        conds.erase(conds.begin() + first, conds.begin() + last);
+    };
+    const bool c128 = amp_bytes == (int)sizeof(double2);
+    for (size_t i = before; i < params.size(); ++i)
+    {
+        out.tensor.push_back(-1);
+        out.butterfly.push_back(-1);
+        BPassParams bp;
+        if (!make_butterfly_params(params[i], amp_bytes, bp))
+            continue;
+        out.butterfly.back() = static_cast<int>(out.bparams.size());
+        out.bparams.push_back(bp);
+    }
+    // automatic mode: below tensor_min_qubits a pass that direct_tensor_pass
+    // did not take runs on the register path. So does a complex128 pass of
+    // Hadamards and mostly phases (a QFT's), whose tensor forms are not even
+    // built: as 8 x 8 stages, where those fit, a replayed QFT flush took 154
+    // us for 172 at 22 qubits and 526 for 544 at 24, but its first flush 1018
+    // for 439 and 1467 for 816 (the host builds both forms); phases on random
+    // pairs between H layers 207 for 222 and 949 for 384 at 22 qubits. Other
+    // passes of mostly phases are priced like any: refused the tensor forms,
+    // six Trotter steps took 933 us for 388 at 22 qubits and 6700 for 2915 at
+    // 25, four QAOA layers 644 for 325 at 22.
     if (tensor_mode == 1 &&
-        (n < tensor_min_qubits(amp_bytes) || (amp_bytes == (int)sizeof(double2) && mostly_phases(q, pp))))
+        (n < tensor_min_qubits(amp_bytes) || (c128 && mostly_phases(q, pp) && hadamards_only(q, pp))))
         tensor_mode = 0;
     double cost4 = 0.0;
     for (size_t i = before; i < params.size(); ++i)
     {
-        out.tensor.push_back(-1);
-        const double creg = register_pass_cost(params[i], amp_bytes);
+        const int bf = out.butterfly[i - before];
+        const double creg = c128 && bf >= 0 ? butterfly_pass_cost(out.bparams[bf]) : register_pass_cost(params[i], amp_bytes);
         double cost = creg;
         if (tensor_mode == 1 || tensor_mode == 2)
         {
@@ -1717,7 +1771,8 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
             {
                 out.tparams.push_back(tp);
                 out.tbuild.push_back(tb);
-                out.tensor.back() = static_cast<int>(out.tparams.size()) - 1;
+                out.tensor[i - before] = static_cast<int>(out.tparams.size()) - 1;
+                out.butterfly[i - before] = -1;
                 cost = ct;
             }
         }
@@ -1726,6 +1781,19 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
     out.cost = cost4;
     if ((tensor_mode != 1 && tensor_mode != 3) || pp.k != kTensorLocal)
         return;
+    if (eight != nullptr)
+    {
+        if (eight->cost < cost4)
+        {
+            drop(before, params.size());
+            out = std::move(*eight);
+        }
+        else
+        {
+            drop(eight_at, before);
+        }
+        return;
+    }
     // the 8 x 8 pieces go behind the others and move down in their place
     PassChoice choice8;
     const size_t end4 = params.size(), tables_before = tables ? tables->size() : 0;
@@ -1733,38 +1801,54 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
         return;
     if (tensor_mode == 1 && choice8.cost >= cost4)
     {
-        params.resize(end4);
-        pieces.resize(end4);
-        conds.resize(end4);
+        drop(end4, params.size());
         if (tables)
             tables->resize(tables_before);
         return;
     }
-    params.erase(params.begin() + before, params.begin() + end4);
-    pieces.erase(pieces.begin() + before, pieces.begin() + end4);
-    conds.erase(conds.begin() + before, conds.begin() + end4);
+    drop(before, end4);
     out = std::move(choice8);
 }
 
-// Complex128 registers below tensor_min_qubits take a pass as 8 x 8 tensor
-// stages from the start, without planning its register form first, when it
-// has at least kSmallTensorOps gates and not mostly multi-qubit phases. Measured on B200, us per
+// Passes that a complex128 register takes as 8 x 8 tensor stages from the
+// start, without planning their register form first.
+//
+// Below tensor_min_qubits: a pass of at least kSmallTensorOps gates that is
+// not mostly multi-qubit phases. Measured on B200, us per
 // flush, register path against 8 x 8 stages: a replayed flush of a 12-layer
 // layered circuit 133 -> 88 at 14 qubits, 185 -> 110 at 17, 231 -> 137 at 19;
 // of an ansatz of depth 4 89 -> 53, 126 -> 86, 172 -> 116. A pass of a few
 // gates stays on the register path: its 7-10 us are less than the launch of
 // its matrix build and its own. (Complex64 keeps its FP32 register path
-// there: its split-TF32 products round more.)
-bool small_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
-                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
-                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out)
+// there: its split-TF32 products round more.) Mostly phases: six Trotter
+// steps replay in 89 for 140 us at 15 qubits and 114 for 169 at 18, but the
+// first flush takes 583 for 478 and 747 for 627, a QFT's 229 for 161 and
+// 598 for 201: most queues are new, so those passes stay too.
+//
+// From tensor_min_qubits on: a pass that costs less as 8 x 8 stages than
+// the least its other forms can cost, so that comparing them could not change
+// the choice (it did not in 400 random circuits of all gates at 20-29 qubits),
+// only take as long again: four QAOA layers at 22 qubits are planned in 0.61
+// ms for 1.21, a layered circuit at 25 in 0.41 for 0.65. Where that does not
+// decide, the form stays in params, pieces, conds and out for
+// choose_execution.
+bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                        std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                        std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out)
 {
-    if (tensor_mode != 1 || amp_bytes != (int)sizeof(double2) || n >= tensor_min_qubits(amp_bytes) ||
-        pp.k != kTensorLocal || pp.ops.size() < kSmallTensorOps)
+    if (tensor_mode != 1 || amp_bytes != (int)sizeof(double2) || pp.k != kTensorLocal)
         return false;
-    if (mostly_phases(q, pp))
+    const bool small = n < tensor_min_qubits(amp_bytes);
+    if (small && (pp.ops.size() < kSmallTensorOps || mostly_phases(q, pp)))
         return false;
-    return build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, out);
+    if (!small && hadamards_only(q, pp))
+        return false;
+    if (!build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, out))
+    {
+        out = PassChoice();
+        return false;
+    }
+    return small || out.cost < cost_floor(q, pp, n);
 }
 
 namespace
@@ -2649,10 +2733,11 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
         }
         std::vector<FPassParams> &params = plan->params;
         const size_t before = params.size();
-        PassChoice choice;
-        const bool small = s.width < 0 && small_tensor_pass(ops, s.pass, n, amp_bytes, tensor_mode_, params, pieces, conds,
-                                                            &plan->tables, choice);
-        if (!small && !build_pieces(ops, s.pass, n, params, nullptr, &pieces, &plan->tables, &conds))
+        PassChoice choice, eight;
+        const bool direct = s.width < 0 && direct_tensor_pass(ops, s.pass, n, amp_bytes, tensor_mode_, params, pieces,
+                                                              conds, &plan->tables, eight);
+        const size_t built = params.size();
+        if (!direct && !build_pieces(ops, s.pass, n, params, nullptr, &pieces, &plan->tables, &conds))
         {
             params.resize(before);
             pieces.resize(before);
@@ -2670,9 +2755,11 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
             tmode = 2;
         else if (s.width == 3 && tensor_mode_ != 0)
             tmode = 3;
-        if (!small)
-            choose_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, before,
-                             tensor_engine_);
+        if (direct)
+            choice = std::move(eight);
+        else
+            choose_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, built,
+                             tensor_engine_, built > before ? &eight : nullptr, before);
         for (size_t i = before; i < params.size(); ++i)
         {
             plan->ks.push_back(pieces[i].k);
@@ -2687,15 +2774,10 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
             {
                 plan->tensor_of.push_back(-1);
             }
-        }
-        // register passes of Hadamard gates and diagonals run as butterflies
-        for (size_t i = before; i < params.size(); ++i)
-        {
-            BPassParams bp;
-            const bool ok = plan->tensor_of[i] < 0 && make_butterfly_params(params[i], amp_bytes, bp);
-            plan->butterfly_of.push_back(ok ? static_cast<int>(plan->bparams.size()) : -1);
-            if (ok)
-                plan->bparams.push_back(bp);
+            const int b = choice.butterfly[i - before];
+            plan->butterfly_of.push_back(b >= 0 ? static_cast<int>(plan->bparams.size()) : -1);
+            if (b >= 0)
+                plan->bparams.push_back(choice.bparams[b]);
         }
         // complex64 register passes read their entries as float2; tensor
         // passes build their matrices from the double2 entries

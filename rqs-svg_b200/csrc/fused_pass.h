@@ -35,7 +35,7 @@ struct StageCond
 constexpr int kTensorLocal = 11;       // local qubits of a tensor pass (2^11-amplitude chunks)
 // Automatic mode: from these sizes on every pass is priced on each path;
 // smaller complex64 registers stay on the register path, smaller complex128
-// ones take 8 x 8 stages by the rule of small_tensor_pass.
+// ones take 8 x 8 stages by the rule of direct_tensor_pass.
 constexpr int kTensorMinQubits = 20;      // complex128
 constexpr int kTensorMinQubitsC64 = 21;   // complex64
 constexpr size_t kSmallTensorOps = 24;    // gates from which a pass of a small register runs as tensor stages
@@ -192,6 +192,9 @@ struct BPassParams
 };
 // False when the pass (entries as double2) has any other gate.
 bool make_butterfly_params(const FPassParams &prm, int amp_bytes, BPassParams &bp);
+bool is_hadamard(const GateOp &op);   // without controls, columns exchanged or not
+// Estimated time of a complex128 butterfly pass in picoseconds per amplitude.
+double butterfly_pass_cost(const BPassParams &bp);
 template <typename R>
 int launch_butterfly_pass(const BPassParams &bp, cudaStream_t stream);
 
@@ -271,21 +274,23 @@ bool build_pieces(const std::vector<GateOp> &q, const PlannedPass &pp, int n, st
                   std::vector<std::vector<FOpSource>> *srcs = nullptr, std::vector<PlannedPass> *pieces = nullptr,
                   std::vector<double2> *tables = nullptr, std::vector<std::vector<StageCond>> *conds = nullptr);
 // How one planned pass runs (choose_execution, fused_pass.cu): per piece an
-// index into tparams / tbuild (a tensor pass) or -1 (the register path), and
+// index into tparams / tbuild (a tensor pass) or -1 (the register path), an
+// index into bparams (a butterfly pass) or -1, and
 // the estimated cost of the whole. engine 1 runs complex64 16 x 16 stages
 // on tcgen05 where a pass allows it, 0 keeps every tensor pass on mma.sync.
 struct PassChoice
 {
-    std::vector<int> tensor;
+    std::vector<int> tensor, butterfly;
     std::vector<TPassParams> tparams;
     std::vector<TBuildParams> tbuild;
+    std::vector<BPassParams> bparams;
     double cost = 0.0;
 };
 void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
                       std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                       std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
-                      size_t before, int engine = 1);
-bool small_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                      size_t before, int engine = 1, PassChoice *eight = nullptr, size_t eight_at = 0);
+bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
                        std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                        std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out);
 int clamp_local_bits(int k, int n);

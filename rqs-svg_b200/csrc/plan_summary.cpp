@@ -92,9 +92,12 @@ void plan_summary(int n, const qcs_b200_gate *gates, uint64_t count, qcs_b200_pl
         std::vector<PlannedPass> pieces;
         std::vector<std::vector<StageCond>> conds;
         // the executor's choice for a complex128 register (automatic mode)
-        PassChoice choice;
-        if (small_tensor_pass(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice))
+        PassChoice choice, eight;
+        const bool direct = direct_tensor_pass(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, eight);
+        const size_t built = params.size();
+        if (direct)
         {
+            choice = std::move(eight);
             out.tensor_eligible += static_cast<uint32_t>(params.size());
         }
         else
@@ -104,14 +107,15 @@ void plan_summary(int n, const qcs_b200_gate *gates, uint64_t count, qcs_b200_pl
                 out.plain_gates += static_cast<uint32_t>(s.pass.ops.size());
                 continue;
             }
-            for (size_t pi = 0; pi < params.size(); ++pi)
+            for (size_t pi = built; pi < params.size(); ++pi)
             {
                 TPassParams tp;
                 TBuildParams tb;
                 if (make_tensor_params(params[pi], conds[pi], 16, tp, tb))
                     ++out.tensor_eligible;
             }
-            choose_execution(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice, 0);
+            choose_execution(queue, s.pass, n, 16, 1, params, pieces, conds, &tables, choice, built, 1,
+                             built > 0 ? &eight : nullptr, 0);
         }
         for (size_t pi = 0; pi < params.size(); ++pi)
         {
