@@ -341,7 +341,9 @@ int qcs_b200_batch_set_tensor_passes(qcs_b200_batch *batch, int mode);
  * How the fused planner (greedy mode, 11 local qubits, 256 gates per pass)
  * would run a gate list on a register of num_qubits, computed on the host
  * without a GPU: for inspecting plans and testing the planner. This entry
- * point has no counterpart in the reference library. Gates are given as in
+ * point has no counterpart in the reference library. (A simulator of up to
+ * 22 qubits runs a queue of at most two launches gate by gate, without the
+ * planner; this reports the planner's passes for every list.) Gates are given as in
  * a batch (any number of targets the API allows); uncontrolled SWAPs only
  * relabel qubits, as in the simulator's fused modes. kinds[] counts the ops
  * of the passes by kind:

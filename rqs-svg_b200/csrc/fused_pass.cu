@@ -2567,8 +2567,18 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
     {
         int launches = 0;
         if (zeros > 0)
+        {
+            double amps = 0.0;
+            for (size_t i = 0; i < zeros; ++i)
+                amps += queued[i].changed_amps(n);
+            if (timer.enabled)
+                timer.begin(stream_, KernelTimer::kPlain, 2.0 * amp_bytes * amps);
             launches += c64 ? launch_collapse_mask<float>(static_cast<float2 *>(state), n, zmask, zval, stream_)
                             : launch_collapse_mask<double>(static_cast<double2 *>(state), n, zmask, zval, stream_);
+            if (timer.enabled)
+                timer.end(stream_);
+            stats.plain_gate_kernels += launches;
+        }
         if (n < fused_min_qubits() && queued.size() - zeros > 1)
         {
             double amps = 0.0;

@@ -1,5 +1,7 @@
 // Host-only view of how the fused planner would run a gate list: passes,
-// stages and pass ops by kind, without a GPU (qcs_b200_plan_summary).
+// stages and pass ops by kind, without a GPU (qcs_b200_plan_summary). The
+// executor asks the planner only for queues of more than two launches
+// (FusedExecutor::run); shorter ones run gate by gate up to 22 qubits.
 #include "fused_pass.h"
 #include "qcs_b200.h"
 

@@ -168,3 +168,25 @@ def test_queues_of_one_or_two_launches(gpu_lib, oracle_lib, n, precision):
     assert bits == ref_bits
     # at most 2 layers and 8 gates of FP32 roundings (6e-8 each) for complex64
     assert np.max(np.abs(state - ref)) <= (1e-12 if precision == 128 else 1e-5)
+
+
+@pytest.mark.parametrize("n", [6, 15])
+def test_collapses_of_short_queues_are_recorded(gpu_lib, n):
+    """Two collapses and a gate run as two plain kernels: both are counted,
+    timed and stand with the bytes of their gates (a collapse changes half of
+    the amplitudes, the H those of the two measured outcomes)."""
+    with qcs_b200.Simulator(gpu_lib, n, n, seed=3, fusion=qcs_b200.FUSION_GREEDY) as sim:
+        sim.run(C.layered_u3_cz(n, 2, seed=n))
+        sim.synchronize()
+        sim.reset_stats()
+        sim.set_kernel_timing(True)
+        for q in (0, 3):
+            sim.measure(q)
+        measures = sim.stats()["kernel_launches"]
+        sim.gate("h", (), (4,), (), ())
+        sim.synchronize()
+        stats, times = sim.stats(), sim.kernel_times()
+    assert stats["kernel_launches"] - measures == 2
+    assert stats["plain_gate_kernels"] == 2 and times["plain_launches"] == 2
+    assert times["plain_ms"] > 0
+    assert times["plain_bytes"] == 2 * 16 * (2 * 2 ** (n - 1) + 2 ** (n - 2))
