@@ -1851,6 +1851,32 @@ bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int
     return small || out.cost < cost_floor(q, pp, n);
 }
 
+// A planned pass built as the executor runs it under a tensor mode. False
+// when it does not fit a pass (nothing is appended then).
+bool build_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                     std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                     std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out, int engine)
+{
+    const size_t before = params.size();
+    PassChoice eight;
+    if (direct_tensor_pass(q, pp, n, amp_bytes, tensor_mode, params, pieces, conds, tables, eight))
+    {
+        out = std::move(eight);
+        return true;
+    }
+    const size_t built = params.size();
+    if (!build_pieces(q, pp, n, params, nullptr, &pieces, tables, &conds))
+    {
+        params.resize(before);
+        pieces.resize(before);
+        conds.resize(before);
+        return false;
+    }
+    choose_execution(q, pp, n, amp_bytes, tensor_mode, params, pieces, conds, tables, out, built, engine,
+                     built > before ? &eight : nullptr, before);
+    return true;
+}
+
 namespace
 {
 
@@ -1969,11 +1995,11 @@ uint64_t fill_local(uint64_t local, int n, int k)
 // Dynamic-programming re-cut of the greedy schedule under the cost model.
 // The greedy passes, concatenated in execution order, form a valid gate
 // order; the planner chooses where to cut it into passes (each cut within
-// kLearnedShift gates of a greedy cut) and, per pass, the block width its
-// stages run with: gate by gate on the register path, or 8 x 8 or 16 x 16
-// tensor stages (the pass is scheduled with three or four dense qubits per
-// stage). Every candidate pass is built as the executor would build it, its
-// features under each width it allows go through the model in one batch,
+// kLearnedShift gates of a greedy cut) and, per pass, how it runs: as the
+// executor itself would run it (build_execution; width -1), or with one block
+// width for all its pieces: gate by gate on the register path, or 8 x 8 or 16
+// x 16 tensor stages. Every candidate pass is built as the executor builds
+// it, its features under each of these go through the model in one batch,
 // and the cover of the gate order with the least predicted time wins. The
 // arithmetic of every gate is the same under any cut; only the grouping
 // changes. Passes keep the greedy plan's number of local qubits.
@@ -1984,7 +2010,7 @@ constexpr int kLearnedShift = 3;
 constexpr double kLearnedMargin = 0.10;
 
 std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vector<Segment> &greedy, int n,
-                                  int amp_bytes, int max_ops, int tensor_mode, CostModel &model,
+                                  int amp_bytes, int max_ops, int tensor_mode, int engine, CostModel &model,
                                   double *predicted_greedy, double *predicted_learned)
 {
     std::vector<Segment> out;
@@ -2031,8 +2057,8 @@ std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vecto
         const int C = static_cast<int>(cuts.size());
 
         // candidates (ci, cj): ops [cuts[ci], cuts[cj]) in one pass, priced
-        // under each block width they allow (feature rows [row0, row1) are
-        // the pieces of one option)
+        // each way it may run (feature rows [row0, row1) are the pieces of
+        // one option; scale is applied to a row's predicted time)
         struct Option
         {
             int ci, cj, width, row0, row1;
@@ -2040,16 +2066,23 @@ std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vecto
         };
         std::vector<Option> opts;
         std::vector<float> feats;
+        std::vector<double> scale;
         std::vector<double2> scratch_tables;
-        auto add_rows = [&](const std::vector<PlannedPass> &pieces, const std::vector<int> &widths,
-                            const std::vector<int> &stages, int ci, int cj, int width, double factor) {
-            Option o{ci, cj, width, static_cast<int>(feats.size() / CostModel::kInputs), 0, factor};
+        // Butterfly passes are recorded as the register passes they are
+        // planned as, which take longer: by the ratio of the two estimates.
+        auto add_rows = [&](const std::vector<FPassParams> &params, const std::vector<PlannedPass> &pieces,
+                            const PassChoice &ch, int ci, int cj, int width, double factor) {
+            Option o{ci, cj, width, static_cast<int>(scale.size()), 0, factor};
             for (size_t i = 0; i < pieces.size(); ++i)
             {
-                const PassFeatures f = pass_features(q, pieces[i], n, widths[i], stages[i]);
+                const int w = ch.tensor[i] >= 0 ? ch.tparams[ch.tensor[i]].width : 1;
+                const PassFeatures f = pass_features(q, pieces[i], n, w, params[i].nstages);
                 feats.insert(feats.end(), f.f, f.f + CostModel::kInputs);
+                scale.push_back(amp_bytes == 16 && ch.butterfly[i] >= 0
+                                    ? butterfly_pass_cost(ch.bparams[ch.butterfly[i]]) / register_pass_cost(params[i], amp_bytes)
+                                    : 1.0);
             }
-            o.row1 = static_cast<int>(feats.size() / CostModel::kInputs);
+            o.row1 = static_cast<int>(scale.size());
             opts.push_back(o);
         };
         for (int ci = 0; ci < C; ++ci)
@@ -2069,68 +2102,38 @@ std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vecto
                 cp.k = K;
                 cp.local = fill_local(d, n, K);
                 cp.ops.assign(seq.begin() + i, seq.begin() + j);
-                std::vector<FPassParams> params;
-                std::vector<PlannedPass> pieces;
-                std::vector<std::vector<StageCond>> conds;
-                scratch_tables.clear();
-                if (!build_pieces(q, cp, n, params, nullptr, &pieces, &scratch_tables, &conds))
-                    continue;
-                std::vector<int> widths(params.size(), 1), stages(params.size());
-                double creg = 0.0, c16 = 0.0, c8 = 0.0;
-                for (size_t pi = 0; pi < params.size(); ++pi)
+                // the executor's own choice, then the others: the model must
+                // predict those faster by more than its error to take them
+                int own = 0;   // the width of all its pieces (0: they differ)
+                for (int width : {-1, 1, 4, 3})
                 {
-                    stages[pi] = params[pi].nstages;
-                    creg += register_pass_cost(params[pi], amp_bytes);
-                }
-                bool ok16 = false, ok8 = false;
-                std::vector<PlannedPass> pieces3;
-                std::vector<int> stages3;
-                if (tensor_ok)
-                {
-                    ok16 = true;
-                    for (size_t pi = 0; pi < params.size() && ok16; ++pi)
+                    if (width == own || (width > 1 && !tensor_ok))
+                        continue;
+                    std::vector<FPassParams> params;
+                    std::vector<PlannedPass> pieces;
+                    std::vector<std::vector<StageCond>> conds;
+                    PassChoice ch;
+                    scratch_tables.clear();
+                    const int mode = width < 0 ? tensor_mode : width == 1 ? 0 : width == 4 ? 2 : 3;
+                    if (!build_execution(q, cp, n, amp_bytes, mode, params, pieces, conds, &scratch_tables, ch, engine))
+                        break;
+                    bool uniform = true, as_asked = true;
+                    for (size_t i = 0; i < pieces.size(); ++i)
                     {
-                        TPassParams tp;
-                        TBuildParams tb;
-                        ok16 = make_tensor_params(params[pi], conds[pi], amp_bytes, tp, tb);
-                        c16 += ok16 ? tensor_pass_cost(tp, amp_bytes) : 0.0;
+                        const int w = ch.tensor[i] >= 0 ? ch.tparams[ch.tensor[i]].width : 1;
+                        uniform = uniform && (i == 0 || w == own);
+                        if (width < 0)
+                            own = w;
+                        as_asked = as_asked && (width < 0 || w == width);
                     }
-                    PlannedPass p3 = cp;
-                    p3.stage_width = 3;
-                    std::vector<FPassParams> params3;
-                    std::vector<std::vector<StageCond>> conds3;
-                    ok8 = build_pieces(q, p3, n, params3, nullptr, &pieces3, &scratch_tables, &conds3);
-                    stages3.resize(params3.size());
-                    for (size_t pi = 0; pi < params3.size() && ok8; ++pi)
-                    {
-                        TPassParams tp;
-                        TBuildParams tb;
-                        ok8 = make_tensor_params(params3[pi], conds3[pi], amp_bytes, tp, tb, 3);
-                        stages3[pi] = params3[pi].nstages;
-                        c8 += ok8 ? tensor_pass_cost(tp, amp_bytes) : 0.0;
-                    }
+                    if (width < 0 && !uniform)
+                        own = 0;
+                    if (as_asked)
+                        add_rows(params, pieces, ch, ci, cj, width, width < 0 ? 1.0 : 1.0 + kLearnedMargin);
                 }
-                // the executor's own choice for this pass (its cost estimate);
-                // the model must predict the others faster by more than its
-                // error to take them
-                int own = 1;
-                double best = creg;
-                if (ok16 && c16 < best)
-                {
-                    own = 4;
-                    best = c16;
-                }
-                if (ok8 && c8 < best)
-                    own = 3;
-                const double other = 1.0 + kLearnedMargin;
-                add_rows(pieces, widths, stages, ci, cj, 1, own == 1 ? 1.0 : other);
-                if (ok16)
-                    add_rows(pieces, std::vector<int>(params.size(), 4), stages, ci, cj, 4, own == 4 ? 1.0 : other);
-                if (ok8)
-                    add_rows(pieces3, std::vector<int>(pieces3.size(), 3), stages3, ci, cj, 3, own == 3 ? 1.0 : other);
             }
         }
-        const int rows = static_cast<int>(feats.size() / CostModel::kInputs);
+        const int rows = static_cast<int>(scale.size());
         std::vector<float> pred(rows);
         if (rows > 0)
             model.predict(feats.data(), rows, pred.data());
@@ -2143,7 +2146,7 @@ std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vecto
         for (size_t o = 0; o < opts.size(); ++o)
         {
             for (int r = opts[o].row0; r < opts[o].row1; ++r)
-                cost[o] += std::exp(double(pred[r])) * amps_ns;
+                cost[o] += std::exp(double(pred[r])) * scale[r] * amps_ns;
             cost[o] *= opts[o].factor;
         }
         // options are grouped by ci ascending, so best[ci] is final when read
@@ -2684,7 +2687,7 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
             else
             {
                 double pg = 0.0, pl = 0.0;
-                segs = plan_learned(ops, segs, n, amp_bytes, max_ops, tensor_mode_, *model_, &pg, &pl);
+                segs = plan_learned(ops, segs, n, amp_bytes, max_ops, tensor_mode_, tensor_engine_, *model_, &pg, &pl);
                 learned_plans_.push_back({key, segs});
             }
         }
@@ -2743,19 +2746,6 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
         }
         std::vector<FPassParams> &params = plan->params;
         const size_t before = params.size();
-        PassChoice choice, eight;
-        const bool direct = s.width < 0 && direct_tensor_pass(ops, s.pass, n, amp_bytes, tensor_mode_, params, pieces,
-                                                              conds, &plan->tables, eight);
-        const size_t built = params.size();
-        if (!direct && !build_pieces(ops, s.pass, n, params, nullptr, &pieces, &plan->tables, &conds))
-        {
-            params.resize(before);
-            pieces.resize(before);
-            conds.resize(before);
-            for (int oi : s.pass.ops)
-                add_step(-1 - (long)oi);
-            continue;
-        }
         // a width the learned planner chose fixes the path (where the pass
         // allows it; else the register path)
         int tmode = tensor_mode_;
@@ -2765,11 +2755,13 @@ int FusedExecutor::run(void *state, int n, int amp_bytes, const std::vector<Gate
             tmode = 2;
         else if (s.width == 3 && tensor_mode_ != 0)
             tmode = 3;
-        if (direct)
-            choice = std::move(eight);
-        else
-            choose_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, built,
-                             tensor_engine_, built > before ? &eight : nullptr, before);
+        PassChoice choice;
+        if (!build_execution(ops, s.pass, n, amp_bytes, tmode, params, pieces, conds, &plan->tables, choice, tensor_engine_))
+        {
+            for (int oi : s.pass.ops)
+                add_step(-1 - (long)oi);
+            continue;
+        }
         for (size_t i = before; i < params.size(); ++i)
         {
             plan->ks.push_back(pieces[i].k);

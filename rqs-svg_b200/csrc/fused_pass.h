@@ -293,6 +293,10 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
 bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
                        std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                        std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out);
+bool build_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                     std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                     std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
+                     int engine = 1);
 int clamp_local_bits(int k, int n);
 // Complex64 passes read their entries as float2: round count double2 entries
 // in place into the first half of the same memory.
