@@ -46,36 +46,158 @@ __global__ void __launch_bounds__(128, sizeof(Real) == 8 ? 3 : 4)
     fused_pass_body<Real, BATCH>(p, [&](const ChunkCtx<V> &cx) { run_stages<V, BATCH>(p, cx); });
 }
 
+using fdev::cmad2;
+using fdev::cmul;
+
+// A complex number in twice the precision, for the entries of stage matrices
+// while gates are applied to them. A matrix serves every group of its stage,
+// so its own rounding does not average out over the register: with entries
+// rounded once, at the end, the state's error of layered circuits is 15-20%
+// smaller (1.43e-15 -> 1.19e-15 at 20 qubits and 12 layers, against 80-bit
+// arithmetic). A build takes 1-2 us longer for it, which working on a
+// matrix's own rows only (below) makes up for.
+struct PairC
+{
+    double2 hi, lo;   // value hi + lo
+};
+
+// s + c of a sum of products, each product's and each addition's rounding
+// error (FMA, Knuth's two-sum) collected in c.
+struct PairSum
+{
+    double s = 0.0, c = 0.0;
+    __device__ __forceinline__ void add(double a, double hi, double lo)
+    {
+        const double p = __dmul_rn(a, hi);
+        const double t = __dadd_rn(s, p), z = __dsub_rn(t, s);
+        const double err = __dadd_rn(__dsub_rn(s, __dsub_rn(t, z)), __dsub_rn(p, z));
+        c = __dadd_rn(c, __dadd_rn(err, __fma_rn(a, lo, __fma_rn(a, hi, -p))));
+        s = t;
+    }
+    __device__ __forceinline__ void put(double &hi, double &lo) const
+    {
+        hi = __dadd_rn(s, c);
+        lo = __dsub_rn(c, __dsub_rn(hi, s));
+    }
+};
+
+struct PairSumC
+{
+    PairSum re, im;
+    __device__ __forceinline__ void add(double2 e, const PairC &x)
+    {
+        re.add(e.x, x.hi.x, x.lo.x);
+        im.add(e.x, x.hi.y, x.lo.y);
+        re.add(-e.y, x.hi.y, x.lo.y);
+        im.add(e.y, x.hi.x, x.lo.x);
+    }
+    __device__ __forceinline__ PairC value() const
+    {
+        PairC r;
+        re.put(r.hi.x, r.lo.x);
+        im.put(r.hi.y, r.lo.y);
+        return r;
+    }
+};
+
+__device__ __forceinline__ PairC cmul(double2 e, const PairC &x)
+{
+    PairSumC a;
+    a.add(e, x);
+    return a.value();
+}
+__device__ __forceinline__ PairC cmad2(double2 e0, const PairC &x0, double2 e1, const PairC &x1)
+{
+    PairSumC a;
+    a.add(e0, x0);
+    a.add(e1, x1);
+    return a.value();
+}
+__device__ __forceinline__ double2 cmad4(const double2 (&e)[4], const double2 (&x)[4])
+{
+    const double2 y = cmad2(e[0], x[0], e[1], x[1]), t = cmad2(e[2], x[2], e[3], x[3]);
+    return make_double2(y.x + t.x, y.y + t.y);
+}
+__device__ __forceinline__ PairC cmad4(const double2 (&e)[4], const PairC (&x)[4])
+{
+    PairSumC a;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        a.add(e[i], x[i]);
+    return a.value();
+}
+__device__ __forceinline__ double2 neg(double2 a) { return make_double2(-a.x, -a.y); }
+__device__ __forceinline__ PairC neg(const PairC &a) { return PairC{neg(a.hi), neg(a.lo)}; }
+// times i, or -i
+__device__ __forceinline__ double2 muli(double2 a, bool minus) { return minus ? make_double2(a.y, -a.x) : make_double2(-a.y, a.x); }
+__device__ __forceinline__ PairC muli(const PairC &a, bool minus) { return PairC{muli(a.hi, minus), muli(a.lo, minus)}; }
+__device__ __forceinline__ void set_real(double2 &a, double v) { a = make_double2(v, 0.0); }
+__device__ __forceinline__ void set_real(PairC &a, double v) { a = PairC{make_double2(v, 0.0), make_double2(0.0, 0.0)}; }
+__device__ __forceinline__ double2 rounded(double2 a) { return a; }
+__device__ __forceinline__ double2 rounded(const PairC &a) { return a.hi; }
+// Im - Re and -(Re + Im)
+__device__ __forceinline__ double2 parts_of(double2 a) { return make_double2(a.y - a.x, -(a.x + a.y)); }
+__device__ __forceinline__ double2 parts_of(const PairC &a)
+{
+    PairSum d, t;
+    d.add(1.0, a.hi.y, a.lo.y);
+    d.add(-1.0, a.hi.x, a.lo.x);
+    t.add(-1.0, a.hi.x, a.lo.x);
+    t.add(-1.0, a.hi.y, a.lo.y);
+    return make_double2(d.s + d.c, t.s + t.c);
+}
+
 // The matrices of a tensor pass: a warp per matrix applies the ops of the
 // matrix's stage to the identity, with the stage's condition bits set as the
 // matrix index says and every other bit outside the stage zero (no op of the
 // stage depends on those). The matrix lives in shared memory, rows in the
 // register stage's slot order, columns in the tensor layout's input slots;
-// the lanes share out (row pair, column) items, an op at a time. It is
-// written as the B fragments of the tensor pass's m16n8k8 products, for the
-// real part Mr, Mi - Mr and -(Mr + Mi): B[u][nu] = M[s(nu)][u] for input slot
+// the lanes share out (row pair, column) items, an op at a time (an 8 x 8
+// matrix's are the rows whose fourth slot bit has its value: one item per
+// lane). It is written as the B fragments of the tensor pass's m16n8k8
+// products, for the real part Mr, Mi - Mr and -(Mr + Mi), for four-product
+// stages Mr, Mi and -Mi: B[u][nu] = M[s(nu)][u] for input slot
 // u (tensor layout) and output column nu = 8i + 2t' + e of n-tile i, output
 // slot s(nu) = 8i + t' + 4e; lane 4g + t of fragment 4 * part + 2j + i holds
 // (B[8j + t][8i + g], B[8j + t + 4][8i + g]).
 // Loops over run-time bits instead of the pass kernel's code unrolled per bit
 // and kind: with a thread per column running that code the build waited on
 // instruction fetches for most of its 17-24 us.
+// An element E is a PairC for a complex128 register's own passes, a double2
+// for complex64 ones and batches (whose matrices are built in every run).
+template <typename E>
 struct MatrixOps
 {
-    double2 (*m)[R];      // [row][column]
+    E (*m)[R];            // [row][column]
     int width;            // log2 of the columns
     uint32_t padmask, padval;   // 8 x 8 stages: the row bit with a fixed value
 
-    // f(row0, row1, column) over the row pairs that differ in bit b
+    // a zero bit inserted into x at the one bit of mask (none: x)
+    static __device__ __forceinline__ uint32_t insert(uint32_t x, uint32_t mask)
+    {
+        const uint32_t lo = x & (mask - 1u);
+        return mask ? lo | ((x ^ lo) << 1) : x;
+    }
+    // row h of those with bit b zero and the pad bit at its value
+    __device__ __forceinline__ uint32_t pair_row(uint32_t h, int b) const
+    {
+        const uint32_t bit = 1u << b;
+        const uint32_t r = bit < padmask ? insert(insert(h, bit), padmask) : insert(insert(h, padmask), bit);
+        return r | padval;
+    }
+
+    // f(row0, row1, column) over the row pairs that differ in bit b. (A group
+    // of one-qubit gates has an identity on the pad bit: nothing to do.)
     template <typename F>
     __device__ __forceinline__ void pairs(int b, uint32_t cm, uint32_t cv, const F &f) const
     {
-        for (int i = threadIdx.x & 31; i < (R / 2) << width; i += 32)
+        if (padmask == 1u << b)
+            return;
+#pragma unroll 1
+        for (int i = threadIdx.x & 31; i < 1 << (2 * width - 1); i += 32)
         {
-            const uint32_t h = static_cast<uint32_t>(i) >> width;
-            const uint32_t lo = h & ((1u << b) - 1u);
-            const uint32_t r = lo | ((h ^ lo) << 1);
-            if ((r & cm) == cv && (r & padmask) == padval)
+            const uint32_t r = pair_row(static_cast<uint32_t>(i) >> width, b);
+            if ((r & cm) == cv)
                 f(r, r | (1u << b), i & ((1 << width) - 1));
         }
         __syncwarp();
@@ -83,10 +205,11 @@ struct MatrixOps
     template <typename F>
     __device__ __forceinline__ void rows(uint32_t cm, uint32_t cv, const F &f) const
     {
-        for (int i = threadIdx.x & 31; i < R << width; i += 32)
+#pragma unroll 1
+        for (int i = threadIdx.x & 31; i < 1 << (2 * width); i += 32)
         {
-            const uint32_t r = static_cast<uint32_t>(i) >> width;
-            if ((r & cm) == cv && (r & padmask) == padval)
+            const uint32_t r = insert(static_cast<uint32_t>(i) >> width, padmask) | padval;
+            if ((r & cm) == cv)
                 f(r, m[r][i & ((1 << width) - 1)]);
         }
         __syncwarp();
@@ -96,7 +219,7 @@ struct MatrixOps
     {
         const double2 e0 = ent[off], e1 = ent[off + 1], e2 = ent[off + 2], e3 = ent[off + 3];
         pairs(b, cm, cv, [&](uint32_t r0, uint32_t r1, int c) {
-            const double2 x0 = m[r0][c], x1 = m[r1][c];
+            const E x0 = m[r0][c], x1 = m[r1][c];
             m[r0][c] = cmad2(e0, x0, e1, x1);
             m[r1][c] = cmad2(e3, x1, e2, x0);
         });
@@ -104,8 +227,8 @@ struct MatrixOps
 };
 
 // One op other than the runs on a matrix.
-template <typename M>
-__device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, const M &ent, uint32_t j0, uint64_t cbase)
+template <typename E, typename M>
+__device__ __forceinline__ void matrix_op(const MatrixOps<E> &w, const FOp &op, const M &ent, uint32_t j0, uint64_t cbase)
 {
     const bool tok = (j0 & op.lcmask) == op.lcval && (cbase & op.gcmask) == op.gcval;
     const uint32_t cm = op.smask, cv = op.sval;
@@ -114,19 +237,21 @@ __device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, con
     switch (op.kind)
     {
     case F_DENSE1:
-    case F_DENSE1R: w.dense1(op.b0, cm, cv, ent, op.moff); break;
+    case F_DENSE1R:
+    case F_DENSE1X2:
     case F_DENSE1X4:
     case F_DENSE1RX4:
-        for (int b = 0; b < kStageBits; ++b)
-            w.dense1(b, 0u, 0u, ent, op.moff + 4 * b);
+    {
+        const bool four = op.kind == F_DENSE1X4 || op.kind == F_DENSE1RX4;
+        const int count = four ? kStageBits : op.kind == F_DENSE1X2 ? 2 : 1;
+#pragma unroll 1
+        for (int i = 0; i < count; ++i)
+            w.dense1(four ? i : i ? op.b1 : op.b0, count == 1 ? cm : 0u, count == 1 ? cv : 0u, ent, op.moff + 4 * i);
         break;
-    case F_DENSE1X2:
-        w.dense1(op.b0, 0u, 0u, ent, op.moff);
-        w.dense1(op.b1, 0u, 0u, ent, op.moff + 4);
-        break;
+    }
     case F_SWAP1:
         w.pairs(op.b0, cm, cv, [&](uint32_t r0, uint32_t r1, int c) {
-            const double2 t = w.m[r0][c];
+            const E t = w.m[r0][c];
             w.m[r0][c] = w.m[r1][c];
             w.m[r1][c] = t;
         });
@@ -148,12 +273,12 @@ __device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, con
             const uint32_t idx[4] = {r, r | (1u << op.b0), r | (1u << op.b1), r | (1u << op.b0) | (1u << op.b1)};
             if (op.kind == F_SWAP2)
             {
-                const double2 t = w.m[idx[1]][c];
+                const E t = w.m[idx[1]][c];
                 w.m[idx[1]][c] = w.m[idx[2]][c];
                 w.m[idx[2]][c] = t;
                 continue;
             }
-            double2 x[4];
+            E x[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 x[q] = w.m[idx[q]][c];
@@ -161,8 +286,8 @@ __device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, con
             for (int q = 0; q < 4; ++q)
             {
                 const int o = op.moff + 4 * q;
-                const double2 y = cmad2(ent[o], x[0], ent[o + 1], x[1]), t = cmad2(ent[o + 2], x[2], ent[o + 3], x[3]);
-                w.m[idx[q]][c] = make_double2(y.x + t.x, y.y + t.y);
+                const double2 e[4] = {ent[o], ent[o + 1], ent[o + 2], ent[o + 3]};
+                w.m[idx[q]][c] = cmad4(e, x);
             }
         }
         __syncwarp();
@@ -171,14 +296,14 @@ __device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, con
     case F_PHASE:
     {
         const double2 e = ent[op.moff];
-        w.rows(cm, cv, [&](uint32_t, double2 &a) { a = cmul(e, a); });
+        w.rows(cm, cv, [&](uint32_t, E &a) { a = cmul(e, a); });
         break;
     }
     case F_MULI:
-        w.rows(cm, cv, [&](uint32_t, double2 &a) { a = op.b1 ? make_double2(a.y, -a.x) : make_double2(-a.y, a.x); });
+        w.rows(cm, cv, [&](uint32_t, E &a) { a = muli(a, op.b1 != 0); });
         break;
     default:
-        w.rows(cm, cv, [&](uint32_t r, double2 &a) {
+        w.rows(cm, cv, [&](uint32_t r, E &a) {
             uint32_t sub = 0;
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -197,10 +322,11 @@ __device__ __forceinline__ void matrix_op(const MatrixOps &w, const FOp &op, con
 
 constexpr int kMatrixWarps = 4;   // matrices per block
 
+template <typename E>
 __global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const __grid_constant__ FPassParams p,
                                                                          const __grid_constant__ TBuildParams tb)
 {
-    __shared__ double2 scratch[kMatrixWarps][R][R];
+    __shared__ E scratch[kMatrixWarps][R][R];
     const int width = tb.width;   // 4: 16 x 16 matrices, 3: 8 x 8
     const int lane = threadIdx.x & 31;
     const uint32_t mat = blockIdx.x * kMatrixWarps + threadIdx.x / 32;
@@ -240,26 +366,26 @@ __global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const _
                 r |= 1u << ((perm >> (2 * b)) & 3);
         return r;
     };
-    double2(*m)[R] = scratch[threadIdx.x / 32];
+    E(*m)[R] = scratch[threadIdx.x / 32];
     for (int i = lane; i < R << width; i += 32)
-        m[i >> width][i & ((1 << width) - 1)] = make_double2(0.0, 0.0);
+        set_real(m[i >> width][i & ((1 << width) - 1)], 0.0);
     __syncwarp();
     if (lane < (1 << width))
-        m[reg(lane)][lane] = make_double2(1.0, 0.0);
+        set_real(m[reg(lane)][lane], 1.0);
     __syncwarp();
-    const MatrixOps w{m, width, padmask, padval};
+    const MatrixOps<E> w{m, width, padmask, padval};
     for (int oi = FS.op_begin; oi < FS.op_end; ++oi)
     {
         const FOp &op = p.ops[oi];
         if (op.kind == F_SIGNS)
         {
-            uint32_t neg = 0;
+            uint32_t flip = 0;
             const int nt = static_cast<int>(op.lcmask);
             for (int i = 1; i <= nt; ++i)
-                neg = sign_term(neg, p.ops[oi + i], j0, cbase);
-            w.rows(0u, 0u, [&](uint32_t r, double2 &a) {
-                if ((neg >> r) & 1)
-                    a = make_double2(-a.x, -a.y);
+                flip = sign_term(flip, p.ops[oi + i], j0, cbase);
+            w.rows(0u, 0u, [&](uint32_t r, E &a) {
+                if ((flip >> r) & 1)
+                    a = neg(a);
             });
             oi += nt;
             continue;
@@ -285,20 +411,20 @@ __global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const _
                     tidx |= 1u << pos;
                 ++pos;
             }
-            double2 E[kStageBits + 1];
-            phase_tables<double2>(E, op, chunk, static_cast<int>(tidx), 1 << (k - kStageBits), p.tables);
+            double2 f[kStageBits + 1];
+            phase_tables<double2>(f, op, chunk, static_cast<int>(tidx), 1 << (k - kStageBits), p.tables);
             const int nterms = static_cast<int>(op.lcmask);
             for (int i = 1; i <= nterms; ++i)
-                phase_term<double2>(E, p.ops[oi + i], j0, cbase, [&](int off) { return ent[off]; });
-            w.rows(0u, 0u, [&](uint32_t r, double2 &a) {
+                phase_term<double2>(f, p.ops[oi + i], j0, cbase, [&](int off) { return ent[off]; });
+            w.rows(0u, 0u, [&](uint32_t r, E &a) {
                 if (op.b1)
                     a = cmul(ent[op.moff + r], a);
                 if (op.b0 & 1)
-                    a = cmul(E[0], a);
+                    a = cmul(f[0], a);
 #pragma unroll
                 for (int b = 0; b < kStageBits; ++b)
                     if (((op.b0 >> (1 + b)) & 1) && ((r >> b) & 1))
-                        a = cmul(E[1 + b], a);
+                        a = cmul(f[1 + b], a);
             });
             oi += nterms;
             continue;
@@ -329,7 +455,7 @@ __global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const _
         for (int i = lane; i < R * R; i += 32)
         {
             const int o = i >> 4, u = i & 15;
-            const double2 y = m[reg(o)][u];
+            const double2 y = rounded(m[reg(o)][u]);
             put(o, u, y.x);
             put(16 + o, u, y.y);
             put(o, 16 + u, -y.y);
@@ -344,8 +470,16 @@ __global__ void __launch_bounds__(32 * kMatrixWarps) stage_matrix_kernel(const _
         for (int i = 0; i < tiles; ++i)
         {
             const uint32_t row = reg(8 * i + (g >> 1) + 4 * (g & 1));
-            const double2 y0 = m[row][8 * j + t], y1 = m[row][8 * j + t + 4];
-            const double parts[3][2] = {{y0.x, y1.x}, {y0.y - y0.x, y1.y - y1.x}, {-(y0.x + y0.y), -(y1.x + y1.y)}};
+            const E &m0 = m[row][8 * j + t], &m1 = m[row][8 * j + t + 4];
+            const double2 y0 = rounded(m0), y1 = rounded(m1), d0 = parts_of(m0), d1 = parts_of(m1);
+            double parts[3][2] = {{y0.x, y1.x}, {d0.x, d1.x}, {d0.y, d1.y}};
+            if (tb.four)
+            {
+                parts[1][0] = y0.y;
+                parts[1][1] = y1.y;
+                parts[2][0] = -y0.y;
+                parts[2][1] = -y1.y;
+            }
 #pragma unroll
             for (int part = 0; part < 3; ++part)
             {
@@ -371,7 +505,10 @@ int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaSt
     const unsigned blocks = (tb.nmats + kMatrixWarps - 1) / kMatrixWarps;
     if (tb.regs == 0)
     {
-        stage_matrix_kernel<<<blocks, threads, 0, stream>>>(prm, tb);
+        if (tb.tf32)
+            stage_matrix_kernel<double2><<<blocks, threads, 0, stream>>>(prm, tb);
+        else
+            stage_matrix_kernel<PairC><<<blocks, threads, 0, stream>>>(prm, tb);
         QCSB_CUDA(cudaGetLastError());
         return 1;
     }
@@ -384,7 +521,7 @@ int launch_stage_matrices(const FPassParams &prm, const TBuildParams &tb, cudaSt
     {
         slice.reg0 = r0;
         const dim3 grid(blocks, std::min<uint32_t>(tb.regs - r0, 65535u));
-        stage_matrix_kernel<<<grid, threads, 0, stream>>>(prm, slice);
+        stage_matrix_kernel<double2><<<grid, threads, 0, stream>>>(prm, slice);
         QCSB_CUDA(cudaGetLastError());
         ++launches;
     }
@@ -1814,7 +1951,13 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
 // start, without planning their register form first.
 //
 // Below tensor_min_qubits: a pass of at least kSmallTensorOps gates that is
-// not mostly multi-qubit phases. Measured on B200, us per
+// not mostly multi-qubit phases, with four real products per complex one:
+// these stages stand in for gates in FP64, and the three-product form rounds
+// 1.35-1.41 times as much as those on layered and matching circuits (at
+// 12-17 qubits, against 80-bit arithmetic), the four-product one with
+// matrices rounded once 0.85-0.98 times. The fourth product takes no time up
+// to 18 qubits, where a pass waits on latencies, and 4-6% of a flush at 19.
+// Measured on B200, us per
 // flush, register path against 8 x 8 stages: a replayed flush of a 12-layer
 // layered circuit 133 -> 88 at 14 qubits, 185 -> 110 at 17, 231 -> 137 at 19;
 // of an ansatz of depth 4 89 -> 53, 126 -> 86, 172 -> 116. A pass of a few
@@ -1848,7 +1991,11 @@ bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int
         out = PassChoice();
         return false;
     }
-    return small || out.cost < cost_floor(q, pp, n);
+    if (!small)
+        return out.cost < cost_floor(q, pp, n);
+    for (size_t j = 0; j < out.tparams.size(); ++j)
+        out.tparams[j].four = out.tbuild[j].four = 1;
+    return true;
 }
 
 // A planned pass built as the executor runs it under a tensor mode. False

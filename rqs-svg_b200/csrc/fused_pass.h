@@ -84,6 +84,9 @@ static_assert(sizeof(TStage) == 28, "TStage layout");
 constexpr int kUmmaSlab = 4096;
 constexpr int kUmmaMaxLocalCond = 1;   // matrices of a stage side by side in N (two at most)
 
+// Up to this many chunks eight warps share one, above four (tensor3_pass_kernel).
+constexpr uint64_t kWideChunks = 256;
+
 struct TBuildParams
 {
     int nstages;
@@ -91,6 +94,7 @@ struct TBuildParams
     int tf32;                    // fragments as TF32 high/low parts (complex64 passes)
     int width;                   // slot bits of the stages: 4 (16 x 16) or 3 (8 x 8)
     int umma;                    // B operands of tcgen05 passes instead of mma.sync fragments
+    int four;                    // fragments of four-product stages: Mr, Mi, -Mi
     double2 *out;                // nmats x kTensorFragments x 32 lanes x 16 bytes (umma: 2 x nmats slabs)
     // batched passes (8 x 8 stages only): registers whose matrices are built
     // (0: one register, entries in the pass parameters); register r reads
@@ -109,6 +113,8 @@ struct TPassParams
     int from_zero;
     int width;                   // 4: 16 x 16 stages, 3: 8 x 8 stages
     int umma;                    // complex64 16 x 16 stages on tcgen05 (tensor_pass_tc.cu)
+    int four;                    // complex128 8 x 8 stages with four real products per complex one (at most
+                                 // kWideChunks chunks)
     uint32_t nmats;              // matrices in mats (umma: the low-part slabs follow the high ones)
     int *err;                    // set to 1 when a tcgen05 pass gives up waiting (host-mapped), or null
     // batched passes (8 x 8 stages only; reg_mats 0: one register): chunk c

@@ -363,7 +363,9 @@ __device__ __forceinline__ StageLayout stage_layout(const TPassParams &p, int st
 template <typename Real, int W>
 constexpr int tensor3_ctas_per_sm() { return W == 4 ? (sizeof(Real) == 8 ? 6 : 8) : 4; }
 
-template <typename Real, int W>
+// FOUR: four real products per complex one. Three round more: their operands
+// are sums of real and imaginary parts, and part of what they add up cancels.
+template <typename Real, int W, bool FOUR = false>
 __global__ void __launch_bounds__(32 * W, tensor3_ctas_per_sm<Real, W>())
     tensor3_pass_kernel(const __grid_constant__ TPassParams p)
 {
@@ -532,12 +534,23 @@ __global__ void __launch_bounds__(32 * W, tensor3_ctas_per_sm<Real, W>())
                 const V x00 = sb[pos(0, 0)], x10 = sb[pos(1, 0)], x01 = sb[pos(0, 1)], x11 = sb[pos(1, 1)];
                 const typename TT::AFrag ar = TT::afrag(x00.x, x10.x, x01.x, x11.x);
                 const typename TT::AFrag ai = TT::afrag(x00.y, x10.y, x01.y, x11.y);
-                const typename TT::AFrag as =
-                    TT::afrag(x00.x + x00.y, x10.x + x10.y, x01.x + x01.y, x11.x + x11.y);
-                // K1 = B0 (Re x + Im x); Re y = K1 + B2 Im x; Im y = K1 + B1 Re x
-                Real k1[4] = {0, 0, 0, 0};
-                TT::mma(k1, as, bf[0]);
-                Real yr[4] = {k1[0], k1[1], k1[2], k1[3]}, yi[4] = {k1[0], k1[1], k1[2], k1[3]};
+                Real yr[4] = {0, 0, 0, 0}, yi[4] = {0, 0, 0, 0};
+                if (FOUR)
+                {
+                    // Re y = B0 Re x + B2 Im x; Im y = B0 Im x + B1 Re x
+                    TT::mma(yr, ar, bf[0]);
+                    TT::mma(yi, ai, bf[0]);
+                }
+                else
+                {
+                    // K1 = B0 (Re x + Im x); Re y = K1 + B2 Im x; Im y = K1 + B1 Re x
+                    const typename TT::AFrag as =
+                        TT::afrag(x00.x + x00.y, x10.x + x10.y, x01.x + x01.y, x11.x + x11.y);
+                    TT::mma(yr, as, bf[0]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        yi[e] = yr[e];
+                }
                 TT::mma(yr, ai, bf[2]);
                 TT::mma(yi, ar, bf[1]);
                 // e = 0: row g, slot t; 1: row g, slot t + 4; 2, 3: row g + 8
@@ -832,7 +845,7 @@ namespace
 {
 
 // Warps per chunk of an 8 x 8 pass (see tensor3_pass_kernel).
-int warps_for(uint64_t chunks) { return chunks <= 256 ? 8 : 4; }
+int warps_for(uint64_t chunks) { return chunks <= kWideChunks ? 8 : 4; }
 
 // One tensor kernel over the pass's chunks, as many CTAs as fit at once.
 template <typename K>
@@ -861,6 +874,12 @@ int launch_tensor_pass(const TPassParams &tp, cudaStream_t stream)
     if (tp.width != 3)
         return launch_chunks(tensor_pass_kernel<R>, kThreads, smem, tp, stream);
     const int w = warps_for(tp.chunks);
+    if (tp.four)
+    {
+        if (w != 8 || sizeof(R) != 8)
+            throw std::runtime_error("internal: four-product passes are complex128 passes of few chunks");
+        return launch_chunks(tensor3_pass_kernel<double, 8, true>, 256, smem, tp, stream);
+    }
     return w == 8 ? launch_chunks(tensor3_pass_kernel<R, 8>, 256, smem, tp, stream)
                   : launch_chunks(tensor3_pass_kernel<R, 4>, 128, smem, tp, stream);
 }
