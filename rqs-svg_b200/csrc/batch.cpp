@@ -410,11 +410,14 @@ void Batch::upload_recipes(size_t first, size_t last, bool tuning)
     reserve(fill_regs_dev_, fill_regs_cap_, regs.size(), tuning);
     reserve(recipes_dev_, recipes_cap_, std::max<size_t>(recipes.size(), 1), tuning);
     reserve(consts_dev_, consts_cap_, consts.size(), tuning);
-    // (the buffers may still be read by the last candidate's fill)
+    // On the batch's stream, behind the last candidate's fill and before the
+    // next one: a plain cudaMemcpy from pageable memory may return before its
+    // data has arrived, and a non-blocking stream does not wait for it.
+    QCSB_CUDA(cudaMemcpyAsync(fill_regs_dev_, regs.data(), sizeof(BatchFillReg) * regs.size(), cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaMemcpyAsync(recipes_dev_, recipes.data(), sizeof(BatchEntry) * recipes.size(), cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaMemcpyAsync(consts_dev_, consts.data(), sizeof(double2) * consts.size(), cudaMemcpyHostToDevice, stream_));
+    // (the vectors go with this function)
     QCSB_CUDA(cudaStreamSynchronize(stream_));
-    QCSB_CUDA(cudaMemcpy(fill_regs_dev_, regs.data(), sizeof(BatchFillReg) * regs.size(), cudaMemcpyHostToDevice));
-    QCSB_CUDA(cudaMemcpy(recipes_dev_, recipes.data(), sizeof(BatchEntry) * recipes.size(), cudaMemcpyHostToDevice));
-    QCSB_CUDA(cudaMemcpy(consts_dev_, consts.data(), sizeof(double2) * consts.size(), cudaMemcpyHostToDevice));
 }
 
 void Batch::upload_params()
@@ -692,8 +695,9 @@ void Batch::build()
     QCSB_CUDA(cudaMalloc(&zpartials_dev_, sizeof(double) * kBatchZPartials * items.size()));
     QCSB_CUDA(cudaMalloc(&zout_dev_, sizeof(double) * zout_count_));
     QCSB_CUDA(cudaMallocHost(&zout_host_, sizeof(double) * zout_count_));
-    QCSB_CUDA(cudaMemcpy(zitems_dev_, items.data(), sizeof(BatchZItem) * items.size(), cudaMemcpyHostToDevice));
-    QCSB_CUDA(cudaMemcpy(zregs_dev_, regs.data(), sizeof(BatchZReg) * regs.size(), cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpyAsync(zitems_dev_, items.data(), sizeof(BatchZItem) * items.size(), cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaMemcpyAsync(zregs_dev_, regs.data(), sizeof(BatchZReg) * regs.size(), cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaStreamSynchronize(stream_));
 
     const size_t param_bytes = sizeof(double) * std::max<size_t>(params_.size(), 1);
     QCSB_CUDA(cudaMalloc(&params_dev_, param_bytes));

@@ -149,7 +149,8 @@ CostModel::CostModel(uint32_t seed)
         p[kW3 + i] = n2(rng);
     QCSB_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     QCSB_CUDA(cudaMalloc(&params_, sizeof(float) * kParams));
-    QCSB_CUDA(cudaMemcpy(params_, p.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpyAsync(params_, p.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaStreamSynchronize(stream_));
     for (int i = 0; i < kIn; ++i)
     {
         in_mean_[i] = 0.0f;
@@ -206,8 +207,8 @@ void CostModel::ensure_batch(int B)
     alloc(&v_, kParams);
     alloc(&scale_, 2);
     QCSB_CUDA(cudaMalloc(&index_, sizeof(int) * B));
-    QCSB_CUDA(cudaMemset(m_, 0, sizeof(float) * kParams));
-    QCSB_CUDA(cudaMemset(v_, 0, sizeof(float) * kParams));
+    QCSB_CUDA(cudaMemsetAsync(m_, 0, sizeof(float) * kParams, stream_));
+    QCSB_CUDA(cudaMemsetAsync(v_, 0, sizeof(float) * kParams, stream_));
     batch_cap_ = B;
 }
 
@@ -289,11 +290,11 @@ float CostModel::train(const float *features, const float *targets, int n, int e
     cudaFree(data_t_);
     QCSB_CUDA(cudaMalloc(&data_x_, sizeof(float) * x.size()));
     QCSB_CUDA(cudaMalloc(&data_t_, sizeof(float) * t.size()));
-    QCSB_CUDA(cudaMemcpy(data_x_, x.data(), sizeof(float) * x.size(), cudaMemcpyHostToDevice));
-    QCSB_CUDA(cudaMemcpy(data_t_, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpyAsync(data_x_, x.data(), sizeof(float) * x.size(), cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaMemcpyAsync(data_t_, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice, stream_));
     ensure_batch(batch);
-    QCSB_CUDA(cudaMemset(m_, 0, sizeof(float) * kParams));
-    QCSB_CUDA(cudaMemset(v_, 0, sizeof(float) * kParams));
+    QCSB_CUDA(cudaMemsetAsync(m_, 0, sizeof(float) * kParams, stream_));
+    QCSB_CUDA(cudaMemsetAsync(v_, 0, sizeof(float) * kParams, stream_));
 
     // capture one training step for this batch size
     if (graph_exec_)
@@ -401,7 +402,8 @@ void CostModel::get_params(float *out) const
 
 void CostModel::set_params(const float *in)
 {
-    QCSB_CUDA(cudaMemcpy(params_, in, sizeof(float) * kParams, cudaMemcpyHostToDevice));
+    QCSB_CUDA(cudaMemcpyAsync(params_, in, sizeof(float) * kParams, cudaMemcpyHostToDevice, stream_));
+    QCSB_CUDA(cudaStreamSynchronize(stream_));
 }
 
 void CostModel::get_scaling(float *out) const

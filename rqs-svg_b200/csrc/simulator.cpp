@@ -183,7 +183,7 @@ void Simulator::allocate_memory()
         QCSB_CUDA(cudaMalloc(&red_partials_, sizeof(double2) * kReduceBlocks));
         injected("cudaMalloc of the reduction ticket");
         QCSB_CUDA(cudaMalloc(&red_ticket_, sizeof(unsigned)));
-        QCSB_CUDA(cudaMemset(red_ticket_, 0, sizeof(unsigned)));
+        QCSB_CUDA(cudaMemsetAsync(red_ticket_, 0, sizeof(unsigned), stream_));
         injected("cudaMalloc of the <Z> partials");
         QCSB_CUDA(cudaMalloc(&zsum_partials_, sizeof(double) * 512 * (kMaxQubits + 1)));
         injected("cudaMalloc of the <Z> sums");
