@@ -355,6 +355,7 @@ int qcs_b200_batch_set_tensor_passes(qcs_b200_batch *batch, int mode);
  *   11 four one-qubit gates (real)    12 phase run (table-fed factors)
  *   13 run of -1 phases               14 one -1 phase of such a run
  *   15 two one-qubit gates (complex)
+ * and in kinds[16] the passes that run as radix-2 butterflies.
  */
 #define QCS_B200_PLAN_KINDS 24
 typedef struct qcs_b200_plan_summary

@@ -130,6 +130,8 @@ void plan_summary(int n, const qcs_b200_gate *gates, uint64_t count, qcs_b200_pl
                 if (choice.tparams[t].width == 3)
                     ++out.tensor8_passes;
             }
+            if (choice.butterfly[pi] >= 0)
+                ++out.kinds[16];
             ++out.passes;
             out.stages += static_cast<uint32_t>(p.nstages);
             out.ops += static_cast<uint32_t>(p.nops);

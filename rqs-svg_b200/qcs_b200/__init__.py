@@ -97,7 +97,7 @@ class BatchGate(ctypes.Structure):
 PLAN_KINDS = 24
 PLAN_KIND_NAMES = {0: "dense1", 1: "x", 2: "dense2", 3: "cswap", 4: "phase", 5: "diag", 6: "term",
                    7: "dense1_real", 9: "phase_i", 10: "group4", 11: "group4_real", 12: "phase_run",
-                   13: "sign_run", 14: "sign_term", 15: "group2"}
+                   13: "sign_run", 14: "sign_term", 15: "group2", 16: "butterfly_pass"}
 
 
 class PlanSummary(ctypes.Structure):

@@ -19,6 +19,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a B200 (runs the CUDA library)")
 
 
+def pytest_collection_modifyitems(items):
+    """The tests against the reference build fail where it was not built (its
+    sources are not everywhere): after all others, so that a run that stops
+    at the first failure has run those."""
+    items.sort(key=lambda item: "test_reference_scale" in item.nodeid or "test_cli_matches_reference_cli" in item.nodeid)
+
+
 @pytest.fixture(scope="session")
 def oracle_lib():
     import qcs_b200

@@ -64,3 +64,41 @@ def test_qft_of_a_basis_state(gpu_lib):
     k = np.arange(1 << n)
     want = np.exp(2j * np.pi * ((x * k) % (1 << n)) / (1 << n)) / np.sqrt(1 << n)
     assert np.max(np.abs(got - want)) <= 1e-14
+
+
+@pytest.mark.parametrize("precision", [128, 64])
+@pytest.mark.parametrize("n", [22, 23])
+def test_qft_with_several_chunks_per_block(gpu_lib, n, precision):
+    """2048 and 4096 chunks on at most 1184 (complex128: 592) blocks, every
+    pass a butterfly; the transform of a basis state in closed form."""
+    circ, x = C.qft(n, seed=n)
+    s = qcs_b200.plan_summary(gpu_lib, n, circ)
+    assert s["kinds"]["butterfly_pass"] == s["passes"]
+    with qcs_b200.Simulator(gpu_lib, n, precision=precision, fusion=qcs_b200.FUSION_GREEDY) as sim:
+        sim.set_tensor_passes(qcs_b200.TENSOR_NEVER)
+        sim.run(circ)
+        got = sim.statevector()
+    k = np.arange(1 << n)
+    want = np.exp(2j * np.pi * ((x * k) % (1 << n)) / (1 << n)) / np.sqrt(1 << n)
+    # relative to the amplitudes, all of one size: n H and n / 2 phases per
+    # amplitude in each precision
+    assert np.max(np.abs(got - want)) * np.sqrt(1 << n) <= (1e-13 if precision == 128 else 1e-4)
+
+
+@pytest.mark.parametrize("precision", [128, 64])
+def test_phases_with_several_chunks_per_block(gpu_lib, oracle_lib, precision):
+    """Stages that hold the low qubits and ones that leave them alone."""
+    n = 22
+    circ = hadamard_phases(n, 5)
+    states = []
+    for lib in (gpu_lib, oracle_lib):
+        kw = {"precision": precision, "fusion": qcs_b200.FUSION_GREEDY} if lib is gpu_lib else {}
+        with qcs_b200.Simulator(lib, n, **kw) as sim:
+            if lib is gpu_lib:
+                sim.set_tensor_passes(qcs_b200.TENSOR_NEVER)
+            sim.set_state("flat")
+            sim.run(circ)
+            states.append(sim.statevector())
+    got, ref = states
+    tol = 1e-12 if precision == 128 else 1e-5
+    assert np.max(np.abs(got - ref)) <= tol * np.max(np.abs(ref))

@@ -47,3 +47,24 @@ def test_phases_with_other_gates_are_priced(gpu_lib, n):
 def test_hadamards_with_phases_stay_butterflies(gpu_lib, n):
     s = qcs_b200.plan_summary(gpu_lib, n, C.qft(n, seed=1)[0])
     assert s["tensor_passes"] == 0
+
+
+@pytest.mark.parametrize("n", [16, 20, 24, 28])
+def test_qft_passes_are_butterflies(gpu_lib, n):
+    s = qcs_b200.plan_summary(gpu_lib, n, C.qft(n, seed=1)[0])
+    assert s["kinds"]["butterfly_pass"] == s["passes"]
+    # a U3 on every qubit in front: passes that hold one are none
+    circ = [("u3", (0.1, 0.2, 0.3), (q,), (), ()) for q in range(n)] + C.qft(n, seed=1)[0]
+    s = qcs_b200.plan_summary(gpu_lib, n, circ)
+    assert 0 < s["kinds"]["butterfly_pass"] + s["tensor_passes"] <= s["passes"]
+    assert s["kinds"]["butterfly_pass"] < s["passes"]
+
+
+@pytest.mark.parametrize("n", [10, 11, 15, 19])
+def test_small_registers_take_8x8_stages(gpu_lib, n):
+    """From 11 qubits (one chunk of a tensor pass) and 24 gates a pass on."""
+    s = qcs_b200.plan_summary(gpu_lib, n, C.layered_u3_cz_cx_toffoli(n, 8, seed=1))
+    assert s["tensor_passes"] == s["tensor8_passes"]
+    assert (s["tensor8_passes"] >= 0.5 * s["passes"]) == (n >= 11)
+    short = [("u3", (0.1, 0.2, 0.3), (q % n,), (), ()) for q in range(23)]
+    assert qcs_b200.plan_summary(gpu_lib, n, short)["tensor_passes"] == 0

@@ -32,3 +32,25 @@ def test_z_sums_match_numpy(gpu_lib, n, precision):
     assert abs(norm / total - 1.0) <= 2.5e-14
     assert np.max(np.abs(z - np.array(want))) <= 5e-14
     assert np.array_equal(z, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [128, 64])
+@pytest.mark.parametrize("n", [20, 21, 22, 25, 26, 27])
+def test_samples_do_not_depend_on_the_qubit_order(gpu_lib, n, precision):
+    """Registers deeper than the sampler's tree (20 levels): the qubits below
+    the leaves on lane bits of the leaf sums (reversed order: all of them up
+    to 25 qubits), above them, and mixed. The outcomes are those of the
+    identity order, which the sequential measurements check; a draw decides
+    otherwise only within the rounding of a state computed in another order,
+    1e-14 of a probability (complex64: 1e-5, one shot in 128 x n draws at
+    most)."""
+    circ = C.layered_u3_cz(n, 1, seed=n)
+    orders = [list(range(n)), list(reversed(range(n))), [int(q) for q in np.random.default_rng(n).permutation(n)]]
+    shots = []
+    for mapping in orders:
+        with qcs_b200.Simulator(gpu_lib, n, precision=precision, mapping=mapping, seed=17) as sim:
+            sim.run(circ)
+            shots.append(sim.sample(128))
+    for other in shots[1:]:
+        assert np.count_nonzero(shots[0] != other) <= (0 if precision == 128 else 1)

@@ -48,3 +48,25 @@ def test_shapes(gpu_lib, oracle_lib, n, low, precision):
     got, ref = states
     tol = 1e-12 if precision == 128 else 1e-5 * np.max(np.abs(ref))
     assert np.max(np.abs(got - ref)) <= tol
+
+
+@pytest.mark.parametrize("precision", [128, 64])
+@pytest.mark.parametrize("low", ["dense", "condition", "untouched"])
+@pytest.mark.parametrize("n", [21, 22])
+def test_shapes_with_several_chunks_per_block(gpu_lib, oracle_lib, n, low, precision):
+    """1024 and 2048 chunks on at most 888 (complex64: 1184) blocks: a block
+    refills its buffer behind the last stage. Tolerances as above."""
+    circ = circuit(n, low, n)
+    states = []
+    for lib in (gpu_lib, oracle_lib):
+        kw = {"precision": precision, "fusion": qcs_b200.FUSION_GREEDY} if lib is gpu_lib else {}
+        with qcs_b200.Simulator(lib, n, **kw) as sim:
+            if lib is gpu_lib:
+                sim.set_tensor_passes(qcs_b200.TENSOR_ALWAYS_8X8)
+            sim.run(circ)
+            states.append(sim.statevector())
+            if lib is gpu_lib:
+                assert sim.stats()["tensor8_passes"] > 0
+    got, ref = states
+    tol = 1e-12 if precision == 128 else 1e-5 * np.max(np.abs(ref))
+    assert np.max(np.abs(got - ref)) <= tol
