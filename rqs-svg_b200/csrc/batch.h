@@ -140,6 +140,7 @@ class Batch
     bool same_structure(const Group &g, const Circuit &c, const std::vector<GateOp> &shape) const;
     void plan_group(Group &g, int k, bool tensor = false);
     void ensure_tensor_mats(size_t first, size_t last);
+    void reserve_for_tuning();
     void layout_entries(size_t first, size_t last, bool tuning);
     void make_recipe(Group &g);
     template <typename T>
