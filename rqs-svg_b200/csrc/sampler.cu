@@ -57,7 +57,7 @@ __device__ __forceinline__ double norm2(V a)
 
 // Leaf sums in physical order, so that the register is read in full lines
 // whatever the measurement order (a register in reversed order, as a QFT's
-// swaps leave it, read a 16-byte amplitude per 4 KiB before: 6.29 -> 0.71 ms at
+// swaps leave it, would read a 16-byte amplitude per 4 KiB: 6.29 -> 0.71 ms at
 // 28 qubits, 6.1 TB/s). Lane l of a warp
 // holds physical bits 0..4; `rest` are the physical bits of the steps below
 // the leaves. A thread adds up the amplitudes that differ in the rest bits

@@ -347,7 +347,7 @@ __device__ __forceinline__ StageLayout stage_layout(const TPassParams &p, int st
 // index (the stage's local condition bits are the lowest group bits, so with
 // at most log2 W of them a warp runs all its tiles with one matrix, fetched
 // before the stage begins).
-// W = 4: six CTAs per SM for complex128 (80 registers; 6 x 32 KiB of chunk),
+// W = 4: six CTAs per SM for complex128 (70 registers; 6 x 32 KiB of chunk),
 // eight for complex64 (64 registers); each step from four measured faster
 // (30-qubit layered and matching complex128: 0.6998 -> 0.6725 -> 0.6551 s and
 // 1.2803 -> 1.2310 -> 1.1979 s at 4, 5, 6). That needs as many chunks: a
@@ -355,6 +355,9 @@ __device__ __forceinline__ StageLayout stage_layout(const TPassParams &p, int st
 // on a nearly idle SM. W = 8 (two tiles per warp) up to 256 chunks: layered
 // circuit 117 -> 106 us at 17 qubits, 143 -> 135 at 19, but 195 -> 214 at 20,
 // 542 -> 612 at 22; 16 warps measured like 8 and worse from 19 qubits on.
+// Batches of 8-256 chunks (11-19 qubits; ansatz, layered and matching
+// circuits) run up to 18% faster with eight than with four, complex128 and
+// complex64 alike; none of 60 was more than 1.5% slower.
 // complex128: the stage layouts are read one stage ahead (the 30-qubit step
 // 594 -> 590 ms) and the last stage stores its outputs straight to the
 // register instead of through shared memory (590 -> 576 ms; 21 qubits 336 ->
@@ -771,9 +774,8 @@ bool make_tensor_params(const FPassParams &prm, const std::vector<StageCond> &co
 // gates of every kind; 280 to 300 passes per path): 8 x 8 stages 2.8 + 1.55
 // per stage (a random-gate pass of four stages 8.8), 16 x 16 stages 2.0 + 3.1
 // per stage, register passes 18-21 ps on the three families and 24 on random
-// gates, of which the former estimate, multiply-adds alone, saw half: the
-// exchanges, predicated gates and the stages' own loads and stores were
-// missing, and passes of few, mixed gates stayed on the register path.
+// gates, half of it multiply-adds, the rest exchanges, predicated gates and
+// the stages' own loads and stores.
 // Complex64 keeps the estimate by multiply-adds (8 x 8 stages 28 units, 16 x
 // 16 ones 30, a register pass's FP32 operations over 0.6): its tensor passes
 // round more than its FP32 gates, so a better estimate of their time would
