@@ -1843,27 +1843,17 @@ double cost_floor(const std::vector<GateOp> &q, const PlannedPass &pp, int n)
 
 } // namespace
 
-// How a planned pass runs: its pieces (built by build_pieces and already
-// appended to params / pieces / conds from index `before` on) on the
-// register path (as butterflies where they are Hadamards and diagonals) or as
-// 16 x 16 tensor stages, per piece whichever the cost
-// estimate favours (tensor mode 1) or 16 x 16 wherever allowed (2); or the
-// same gates replanned with three dense bits per stage as 8 x 8 tensor
-// stages, which then replace those pieces: when the estimate favours them
-// (1) or wherever every piece allows them (3). eight: the 8 x 8 form where
-// direct_tensor_pass left it, its pieces from index eight_at to `before`.
-void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
-                      std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
-                      std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
-                      size_t before, int engine, PassChoice *eight, size_t eight_at)
+namespace
+{
+
+// The pieces from index `before` on without an 8 x 8 form: on the register
+// path (as butterflies where they are Hadamards and diagonals) or as 16 x 16
+// stages. Returns the tensor mode that is left for the pass.
+int price_pieces(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                 const std::vector<FPassParams> &params, const std::vector<std::vector<StageCond>> &conds, size_t before,
+                 int engine, PassChoice &out)
 {
     out = PassChoice();
-    // drops pieces [first, last)
-    auto drop = [&](size_t first, size_t last) {
-        params.erase(params.begin() + first, params.begin() + last);
-        pieces.erase(pieces.begin() + first, pieces.begin() + last);
-        conds.erase(conds.begin() + first, conds.begin() + last);
-    };
     const bool c128 = amp_bytes == (int)sizeof(double2);
     for (size_t i = before; i < params.size(); ++i)
     {
@@ -1916,11 +1906,37 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
         cost4 += cost;
     }
     out.cost = cost4;
+    return tensor_mode;
+}
+
+} // namespace
+
+// How a planned pass runs: its pieces (built by build_pieces and already
+// appended to params / pieces / conds from index `before` on) on the
+// register path (as butterflies where they are Hadamards and diagonals) or as
+// 16 x 16 tensor stages, per piece whichever the cost
+// estimate favours (tensor mode 1) or 16 x 16 wherever allowed (2); or the
+// same gates replanned with three dense bits per stage as 8 x 8 tensor
+// stages, which then replace those pieces: when the estimate favours them
+// (1) or wherever every piece allows them (3). eight: the 8 x 8 form where
+// direct_tensor_pass left it, its pieces from index eight_at to `before`.
+void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
+                      std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
+                      std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out,
+                      size_t before, int engine, PassChoice *eight, size_t eight_at)
+{
+    tensor_mode = price_pieces(q, pp, n, amp_bytes, tensor_mode, params, conds, before, engine, out);
+    // drops pieces [first, last)
+    auto drop = [&](size_t first, size_t last) {
+        params.erase(params.begin() + first, params.begin() + last);
+        pieces.erase(pieces.begin() + first, pieces.begin() + last);
+        conds.erase(conds.begin() + first, conds.begin() + last);
+    };
     if ((tensor_mode != 1 && tensor_mode != 3) || pp.k != kTensorLocal)
         return;
     if (eight != nullptr)
     {
-        if (eight->cost < cost4)
+        if (eight->cost < out.cost)
         {
             drop(before, params.size());
             out = std::move(*eight);
@@ -1936,7 +1952,7 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
     const size_t end4 = params.size(), tables_before = tables ? tables->size() : 0;
     if (!build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, choice8))
         return;
-    if (tensor_mode == 1 && choice8.cost >= cost4)
+    if (tensor_mode == 1 && choice8.cost >= out.cost)
     {
         drop(end4, params.size());
         if (tables)
@@ -1975,23 +1991,35 @@ void choose_execution(const std::vector<GateOp> &q, const PlannedPass &pp, int n
 // ms for 1.21, a layered circuit at 25 in 0.41 for 0.65. Where that does not
 // decide, the form stays in params, pieces, conds and out for
 // choose_execution.
+enum class Eight
+{
+    kNo,      // the other forms come first
+    kAlways,  // where it can be built
+    kFloor,   // where it costs less than cost_floor
+};
+
+static Eight eight_first(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode)
+{
+    if (tensor_mode != 1 || amp_bytes != (int)sizeof(double2) || pp.k != kTensorLocal)
+        return Eight::kNo;
+    if (n < tensor_min_qubits(amp_bytes))
+        return pp.ops.size() < kSmallTensorOps || mostly_phases(q, pp) ? Eight::kNo : Eight::kAlways;
+    return hadamards_only(q, pp) ? Eight::kNo : Eight::kFloor;
+}
+
 bool direct_tensor_pass(const std::vector<GateOp> &q, const PlannedPass &pp, int n, int amp_bytes, int tensor_mode,
                         std::vector<FPassParams> &params, std::vector<PlannedPass> &pieces,
                         std::vector<std::vector<StageCond>> &conds, std::vector<double2> *tables, PassChoice &out)
 {
-    if (tensor_mode != 1 || amp_bytes != (int)sizeof(double2) || pp.k != kTensorLocal)
-        return false;
-    const bool small = n < tensor_min_qubits(amp_bytes);
-    if (small && (pp.ops.size() < kSmallTensorOps || mostly_phases(q, pp)))
-        return false;
-    if (!small && hadamards_only(q, pp))
+    const Eight first = eight_first(q, pp, n, amp_bytes, tensor_mode);
+    if (first == Eight::kNo)
         return false;
     if (!build_tensor8(q, pp, n, amp_bytes, params, pieces, conds, tables, out))
     {
         out = PassChoice();
         return false;
     }
-    if (!small)
+    if (first == Eight::kFloor)
         return out.cost < cost_floor(q, pp, n);
     for (size_t j = 0; j < out.tparams.size(); ++j)
         out.tparams[j].four = out.tbuild[j].four = 1;
@@ -2143,10 +2171,10 @@ uint64_t fill_local(uint64_t local, int n, int k)
 // The greedy passes, concatenated in execution order, form a valid gate
 // order; the planner chooses where to cut it into passes (each cut within
 // kLearnedShift gates of a greedy cut) and, per pass, how it runs: as the
-// executor itself would run it (build_execution; width -1), or with one block
+// executor itself would run it (as build_execution chooses; width -1), or with one block
 // width for all its pieces: gate by gate on the register path, or 8 x 8 or 16
 // x 16 tensor stages. Every candidate pass is built as the executor builds
-// it, its features under each of these go through the model in one batch,
+// it, each form once, its features under each of these go through the model in one batch,
 // and the cover of the gate order with the least predicted time wins. The
 // arithmetic of every gate is the same under any cut; only the grouping
 // changes. Passes keep the greedy plan's number of local qubits.
@@ -2249,35 +2277,44 @@ std::vector<Segment> plan_learned(const std::vector<GateOp> &q, const std::vecto
                 cp.k = K;
                 cp.local = fill_local(d, n, K);
                 cp.ops.assign(seq.begin() + i, seq.begin() + j);
+                // the pass's forms, each built once: 8 x 8 stages, and the
+                // pieces for the register path or 16 x 16 stages
+                std::vector<FPassParams> params, params8;
+                std::vector<PlannedPass> pieces, pieces8;
+                std::vector<std::vector<StageCond>> conds, conds8;
+                PassChoice reg, own4, all16, eight;
+                scratch_tables.clear();
+                const Eight first = eight_first(q, cp, n, amp_bytes, tensor_mode);
+                const bool have8 = K == kTensorLocal && (tensor_ok || first != Eight::kNo) &&
+                                   build_tensor8(q, cp, n, amp_bytes, params8, pieces8, conds8, &scratch_tables, eight);
+                if (!build_pieces(q, cp, n, params, nullptr, &pieces, &scratch_tables, &conds))
+                    continue;
+                const int mode = price_pieces(q, cp, n, amp_bytes, tensor_mode, params, conds, 0, engine, own4);
+                // what build_execution comes to
+                const bool own8 = have8 && (first == Eight::kAlways || mode == 3 || (mode == 1 && eight.cost < own4.cost));
                 // the executor's own choice, then the others: the model must
                 // predict those faster by more than its error to take them
-                int own = 0;   // the width of all its pieces (0: they differ)
-                for (int width : {-1, 1, 4, 3})
+                const double other = 1.0 + kLearnedMargin;
+                const int own = own8 ? 3 : own4.tparams.empty() ? 1 : own4.tparams.size() == params.size() ? 4 : 0;
+                if (own8)
+                    add_rows(params8, pieces8, eight, ci, cj, -1, 1.0);
+                else
+                    add_rows(params, pieces, own4, ci, cj, -1, 1.0);
+                if (own != 1 && own4.tparams.empty())
+                    add_rows(params, pieces, own4, ci, cj, 1, other);
+                else if (own != 1)
                 {
-                    if (width == own || (width > 1 && !tensor_ok))
-                        continue;
-                    std::vector<FPassParams> params;
-                    std::vector<PlannedPass> pieces;
-                    std::vector<std::vector<StageCond>> conds;
-                    PassChoice ch;
-                    scratch_tables.clear();
-                    const int mode = width < 0 ? tensor_mode : width == 1 ? 0 : width == 4 ? 2 : 3;
-                    if (!build_execution(q, cp, n, amp_bytes, mode, params, pieces, conds, &scratch_tables, ch, engine))
-                        break;
-                    bool uniform = true, as_asked = true;
-                    for (size_t i = 0; i < pieces.size(); ++i)
-                    {
-                        const int w = ch.tensor[i] >= 0 ? ch.tparams[ch.tensor[i]].width : 1;
-                        uniform = uniform && (i == 0 || w == own);
-                        if (width < 0)
-                            own = w;
-                        as_asked = as_asked && (width < 0 || w == width);
-                    }
-                    if (width < 0 && !uniform)
-                        own = 0;
-                    if (as_asked)
-                        add_rows(params, pieces, ch, ci, cj, width, width < 0 ? 1.0 : 1.0 + kLearnedMargin);
+                    price_pieces(q, cp, n, amp_bytes, 0, params, conds, 0, engine, reg);
+                    add_rows(params, pieces, reg, ci, cj, 1, other);
                 }
+                if (tensor_ok && own != 4)
+                {
+                    price_pieces(q, cp, n, amp_bytes, 2, params, conds, 0, engine, all16);
+                    if (all16.tparams.size() == params.size())
+                        add_rows(params, pieces, all16, ci, cj, 4, other);
+                }
+                if (have8 && tensor_ok && own != 3)
+                    add_rows(params8, pieces8, eight, ci, cj, 3, other);
             }
         }
         const int rows = static_cast<int>(scale.size());
